@@ -1628,92 +1628,167 @@ template <int LPL, int LPW> __device__ __forceinline__ double slot_reduce64(doub
     return a;
 }
 
+// Four columns of one link or of a group of links (their products summed
+// plainly) into the compensated sums.
+__device__ __forceinline__ void link_add1(KSum *acc, float c, float4 q) {
+    kmul_add(acc[0], c, q.x); kmul_add(acc[1], c, q.y); kmul_add(acc[2], c, q.z); kmul_add(acc[3], c, q.w);
+}
+__device__ __forceinline__ void link_add2(KSum *acc, const float *c, const float4 *q) {
+    kgroup_add(acc[0], fmaf(c[1], q[1].x, c[0] * q[0].x));
+    kgroup_add(acc[1], fmaf(c[1], q[1].y, c[0] * q[0].y));
+    kgroup_add(acc[2], fmaf(c[1], q[1].z, c[0] * q[0].z));
+    kgroup_add(acc[3], fmaf(c[1], q[1].w, c[0] * q[0].w));
+}
+__device__ __forceinline__ void link_add4(KSum *acc, const float *c, const float4 *q) {
+    kgroup_add(acc[0], fmaf(c[3], q[3].x, fmaf(c[2], q[2].x, fmaf(c[1], q[1].x, c[0] * q[0].x))));
+    kgroup_add(acc[1], fmaf(c[3], q[3].y, fmaf(c[2], q[2].y, fmaf(c[1], q[1].y, c[0] * q[0].y))));
+    kgroup_add(acc[2], fmaf(c[3], q[3].z, fmaf(c[2], q[2].z, fmaf(c[1], q[1].z, c[0] * q[0].z))));
+    kgroup_add(acc[3], fmaf(c[3], q[3].w, fmaf(c[2], q[2].w, fmaf(c[1], q[1].w, c[0] * q[0].w))));
+}
+// U links of a slot, LPW apart: the link words, then the charge gathers, all
+// issued before any is used; a link past the row's end is a zero
+template <int U, int LPL, int LPW, bool FULL>
+__device__ __forceinline__ void load_links(const uint32_t *__restrict__ src, const float *__restrict__ coef,
+                                           const float4 *__restrict__ Q4, int l, int e, int ri, float *c, float4 *q) {
+    uint32_t j[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const bool ok = FULL || l + u * LPW < e;
+        c[u] = ok ? __ldcs(&coef[l + u * LPW]) : 0.f;
+        j[u] = ok ? __ldcs(&src[l + u * LPW]) & kSrcMask : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        if (FULL || l + u * LPW < e) q[u] = Q4[(int64_t)j[u] * LPL + ri];
+        else q[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
 // Link product for K = 4, 8, ..., 32 right-hand sides, mixed: K/4 lanes
 // share a link and each owns four right-hand sides (one 16-byte charge
 // gather per link); a warp has 32/(K/4) link slots (lanes beyond them idle).
 // CTA b owns the contiguous rows [row_split[b], row_split[b+1]) (split for
-// equal link counts), its warps take every eighth row: consecutive rows
-// share most of their sources, so the gathers hit L1.
+// equal work), its warps take every eighth row: consecutive rows share most
+// of their sources, so the gathers hit L1.
+//
+// Bound by the latency of the charge gathers (72 % of a warp's time; L1's
+// wavefront rate at 67 %, DRAM at 14 %; the time falls in proportion to the
+// warps in flight up to six CTAs an SM). So a slot keeps as many gathers in
+// flight as pays for the occupancy its registers cost: eight from 16 columns
+// on (four CTAs an SM), four for 8 and 12 columns (six), two for 4 (seven;
+// its rows are short); the odd links at a row's end are loaded together; and
+// the next row's offsets and link words come into L1 and L2 while a row is
+// summed. Each slot adds its links in the same order and grouping at every
+// width of the passes. Microseconds a launch, before (four per pass from 16
+// columns on, two below) and after, with k_row_split's row weight: 28.5M
+// links 24 columns 290 -> 267, 32 columns 330 -> 291; dielectric slab, 20M
+// links, 16 columns 212 -> 138; 11.6M, 20 columns 138 -> 116; 11M, 12
+// columns 116 -> 107; 3.4M, 8 columns 50.5 -> 38.4; 1.1M, 4 columns 24.2 ->
+// 20.2. Slower: chunks of link words loaded one per lane and handed to the
+// slots by shuffle (349 at 24 columns), a row's first links loaded a row
+// ahead into registers (310), source and coefficient interleaved in 8-byte
+// words (292), CTAs of 512 to 1024 threads on one row range (294 at best).
 template <int K>
-__global__ void __launch_bounds__(256) k_spmv32_multi(const int32_t *__restrict__ row_split, const int64_t *__restrict__ ptr,
-                                                      const uint32_t *__restrict__ src, const float *__restrict__ coef,
-                                                      const float *__restrict__ Q, float2 *__restrict__ P) {
+__global__ void __launch_bounds__(256, K >= 16 ? 4 : (K >= 8 ? 6 : 7))
+    k_spmv32_multi(const int32_t *__restrict__ row_split, const int64_t *__restrict__ ptr, const uint32_t *__restrict__ src,
+                   const float *__restrict__ coef, const float *__restrict__ Q, float2 *__restrict__ P) {
     constexpr int LPL = K / 4, LPW = 32 / LPL;
     // from 20 columns on (at most six slots) a row's slot sums meet in shared
     // memory: lane c < K adds the slots' (sum, correction) pairs of column c
     // in slot order and writes it (fewer instructions than the shuffle tree;
     // with eight or more slots the extra shared-memory wavefronts cost more
-    // than they save: 16-column slab product 0.538 -> 0.593 ms)
+    // than they save: 16-column slab product 0.538 -> 0.593 ms). Sums and
+    // corrections are separate arrays: no bank conflicts on either side.
     constexpr bool SMEM_RED = K >= 20;
-    __shared__ __align__(16) KSum red[SMEM_RED ? 8 : 1][SMEM_RED ? LPW * K : 1];
-    int lane = threadIdx.x & 31, li = lane / LPL, ri = lane % LPL;
-    KSum *wred = red[SMEM_RED ? (threadIdx.x >> 5) : 0];
-    bool slot_ok = li < LPW;
+    __shared__ __align__(16) float red[SMEM_RED ? 8 : 1][SMEM_RED ? 2 * LPW * K : 1];
+    const int lane = threadIdx.x & 31, li = lane / LPL, ri = lane % LPL;
+    float *wred = red[SMEM_RED ? (threadIdx.x >> 5) : 0];
+    const bool slot_ok = li < LPW;
     const float4 *Q4 = reinterpret_cast<const float4 *>(Q);
-    int r0 = row_split[blockIdx.x], r1 = row_split[blockIdx.x + 1];
-    for (int row = r0 + (threadIdx.x >> 5); row < r1; row += 8) {
+    const int r1 = row_split[blockIdx.x + 1];
+    int row = row_split[blockIdx.x] + (threadIdx.x >> 5);
+    if (row >= r1) return;
+    int s = (int)ptr[row], e = (int)ptr[row + 1];
+    while (true) {
         KSum acc[4];
 #pragma unroll
         for (int r = 0; r < 4; r++) { acc[r].s = 0.f; acc[r].c = 0.f; }
-        int s = (int)ptr[row], e = (int)ptr[row + 1];
+        int ns = 0, ne = 0;  // the warp's next row
+        if (row + 8 < r1) { ns = (int)ptr[row + 8]; ne = (int)ptr[row + 9]; }
         int l = s + li;
+        // the next row's link words (up to 1024 links) into L2
+        auto prefetch_next = [&]() {
+            const int o = ns + 32 * lane;
+            if (o < ne) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(coef + o));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(src + o));
+            }
+        };
         if (slot_ok) {
             if constexpr (K >= 16) {
-                // four links per slot and pass (four charge gathers in flight
-                // per lane), their products summed plainly, then added to
-                // the compensated sums (served 22-column requests: 1.5 %
-                // faster than two per pass)
+                // groups of four links are summed plainly, then added to the
+                // compensated sums; of a slot's last three, two are such a
+                // group and the third is its own update
+                for (; l + 7 * LPW < e; l += 8 * LPW) {
+                    float c[8];
+                    float4 q[8];
+                    load_links<8, LPL, LPW, true>(src, coef, Q4, l, e, ri, c, q);
+                    link_add4(acc, c, q);
+                    link_add4(acc, c + 4, q + 4);
+                }
                 for (; l + 3 * LPW < e; l += 4 * LPW) {
-                    float c0 = __ldcs(&coef[l]), c1 = __ldcs(&coef[l + LPW]);
-                    float c2 = __ldcs(&coef[l + 2 * LPW]), c3 = __ldcs(&coef[l + 3 * LPW]);
-                    uint32_t j0 = __ldcs(&src[l]) & kSrcMask, j1 = __ldcs(&src[l + LPW]) & kSrcMask;
-                    uint32_t j2 = __ldcs(&src[l + 2 * LPW]) & kSrcMask, j3 = __ldcs(&src[l + 3 * LPW]) & kSrcMask;
-                    float4 q0 = Q4[(int64_t)j0 * LPL + ri], q1 = Q4[(int64_t)j1 * LPL + ri];
-                    float4 q2 = Q4[(int64_t)j2 * LPL + ri], q3 = Q4[(int64_t)j3 * LPL + ri];
-                    kgroup_add(acc[0], fmaf(c3, q3.x, fmaf(c2, q2.x, fmaf(c1, q1.x, c0 * q0.x))));
-                    kgroup_add(acc[1], fmaf(c3, q3.y, fmaf(c2, q2.y, fmaf(c1, q1.y, c0 * q0.y))));
-                    kgroup_add(acc[2], fmaf(c3, q3.z, fmaf(c2, q2.z, fmaf(c1, q1.z, c0 * q0.z))));
-                    kgroup_add(acc[3], fmaf(c3, q3.w, fmaf(c2, q2.w, fmaf(c1, q1.w, c0 * q0.w))));
+                    float c[4];
+                    float4 q[4];
+                    load_links<4, LPL, LPW, true>(src, coef, Q4, l, e, ri, c, q);
+                    link_add4(acc, c, q);
                 }
-            }
-            // two links per slot and pass; from 16 columns on (issue bound)
-            // their products are summed plainly, then added to the
-            // compensated sums (kgroup_add), below that each is (kmul_add)
-            for (; l + LPW < e; l += 2 * LPW) {
-                float c0 = __ldcs(&coef[l]), c1 = __ldcs(&coef[l + LPW]);
-                uint32_t j0 = __ldcs(&src[l]) & kSrcMask, j1 = __ldcs(&src[l + LPW]) & kSrcMask;
-                float4 q0 = Q4[(int64_t)j0 * LPL + ri], q1 = Q4[(int64_t)j1 * LPL + ri];
-                if constexpr (K >= 16) {
-                    kgroup_add(acc[0], fmaf(c1, q1.x, c0 * q0.x));
-                    kgroup_add(acc[1], fmaf(c1, q1.y, c0 * q0.y));
-                    kgroup_add(acc[2], fmaf(c1, q1.z, c0 * q0.z));
-                    kgroup_add(acc[3], fmaf(c1, q1.w, c0 * q0.w));
-                } else {
-                    kmul_add(acc[0], c0, q0.x); kmul_add(acc[1], c0, q0.y); kmul_add(acc[2], c0, q0.z); kmul_add(acc[3], c0, q0.w);
-                    kmul_add(acc[0], c1, q1.x); kmul_add(acc[1], c1, q1.y); kmul_add(acc[2], c1, q1.z); kmul_add(acc[3], c1, q1.w);
+                prefetch_next();
+                float c[3];
+                float4 q[3];
+                load_links<3, LPL, LPW, false>(src, coef, Q4, l, e, ri, c, q);
+                const bool two = l + LPW < e;
+                if (two) link_add2(acc, c, q);
+                if (two ? l + 2 * LPW < e : l < e) link_add1(acc, two ? c[2] : c[0], two ? q[2] : q[0]);
+            } else {
+                // below 16 columns every link is an update of its own
+                if constexpr (K >= 8) {
+                    for (; l + 3 * LPW < e; l += 4 * LPW) {
+                        float c[4];
+                        float4 q[4];
+                        load_links<4, LPL, LPW, true>(src, coef, Q4, l, e, ri, c, q);
+#pragma unroll
+                        for (int u = 0; u < 4; u++) link_add1(acc, c[u], q[u]);
+                    }
+                    prefetch_next();
                 }
-            }
-            if (l < e) {
-                float c0 = __ldcs(&coef[l]);
-                uint32_t j0 = __ldcs(&src[l]) & kSrcMask;
-                float4 q0 = Q4[(int64_t)j0 * LPL + ri];
-                kmul_add(acc[0], c0, q0.x); kmul_add(acc[1], c0, q0.y); kmul_add(acc[2], c0, q0.z); kmul_add(acc[3], c0, q0.w);
+                for (; l + LPW < e; l += 2 * LPW) {
+                    float c[2];
+                    float4 q[2];
+                    load_links<2, LPL, LPW, true>(src, coef, Q4, l, e, ri, c, q);
+                    link_add1(acc, c[0], q[0]);
+                    link_add1(acc, c[1], q[1]);
+                }
+                if (l < e) {
+                    float c[1];
+                    float4 q[1];
+                    load_links<1, LPL, LPW, true>(src, coef, Q4, l, e, ri, c, q);
+                    link_add1(acc, c[0], q[0]);
+                }
             }
         }
         if constexpr (SMEM_RED) {
             if (slot_ok) {
-                float4 *o = reinterpret_cast<float4 *>(wred + li * K + 4 * ri);
-                o[0] = make_float4(acc[0].s, acc[0].c, acc[1].s, acc[1].c);
-                o[1] = make_float4(acc[2].s, acc[2].c, acc[3].s, acc[3].c);
+                float *o = wred + li * K + 4 * ri;
+                *reinterpret_cast<float4 *>(o) = make_float4(acc[0].s, acc[1].s, acc[2].s, acc[3].s);
+                *reinterpret_cast<float4 *>(o + LPW * K) = make_float4(acc[0].c, acc[1].c, acc[2].c, acc[3].c);
             }
             __syncwarp();
             if (lane < K) {
-                KSum a = wred[lane];
+                KSum a = {wred[lane], wred[LPW * K + lane]};
 #pragma unroll
                 for (int q = 1; q < LPW; q++) {
-                    const KSum b = wred[q * K + lane];
-                    a.c += b.c;
-                    kadd(a, b.s);
+                    a.c += wred[(LPW + q) * K + lane];
+                    kadd(a, wred[q * K + lane]);
                 }
                 P[(int64_t)row * K + lane] = make_float2(a.s, a.c);
             }
@@ -1727,6 +1802,10 @@ __global__ void __launch_bounds__(256) k_spmv32_multi(const int32_t *__restrict_
                 out[1] = make_float4(acc[2].s, acc[2].c, acc[3].s, acc[3].c);
             }
         }
+        row += 8;
+        if (row >= r1) return;
+        s = ns;
+        e = ne;
     }
 }
 
@@ -3058,8 +3137,15 @@ __global__ void k_chains(int nb, const int32_t *__restrict__ broot, const int32_
     }
 }
 
-// Contiguous row ranges of about equal work (links + 8 per row): the first
-// row whose work offset reaches b/nb of the total (a binary search per range)
+// Contiguous row ranges of about equal work: the first row whose work offset
+// reaches b/nb of the total (a binary search per range). A row costs its
+// links and about as long as kRowWork links for its own chain (offsets, first
+// words, reduction, store): half of a model's rows are leaves of some 20
+// links, and ranges weighted 8 a row left the last CTAs running alone (20M
+// links, 16 columns 212 -> 195 us by this alone; 16 to 64 are equal within
+// 2 %).
+static const double kRowWork = 32.0;
+static const int64_t kMinRangeRows = 16;  // small models: two rows a warp before fewer CTAs (1.1M links, 4 columns 24.2 -> 20.2 us)
 __global__ void k_row_split(int64_t Nn, const int64_t *__restrict__ ptr, int64_t nb, double total, int32_t *split) {
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b <= nb; b += (int64_t)gridDim.x * blockDim.x) {
         if (b == 0 || b == nb) {
@@ -3070,25 +3156,25 @@ __global__ void k_row_split(int64_t Nn, const int64_t *__restrict__ ptr, int64_t
         int64_t lo = 0, hi = Nn;
         while (lo < hi) {
             int64_t m = lo + ((hi - lo) >> 1);
-            if ((double)ptr[m] + 8.0 * (double)m < target) lo = m + 1;
+            if ((double)ptr[m] + kRowWork * (double)m < target) lo = m + 1;
             else hi = m;
         }
         split[b] = (int32_t)lo;
     }
 }
 
-// Contiguous row ranges of about equal work (links + 8 per row) for the
-// multi-right-hand-side link product: ctas ranges (capped so that each has at
-// least 64 rows).
+// Contiguous row ranges of about equal work for the multi-right-hand-side
+// link product: ctas ranges (capped so that each has at least kMinRangeRows
+// rows on average).
 static int set_row_split(DeviceProblem *p, int64_t ctas) {
     int64_t Nn = p->Nn, L = p->L;
-    int64_t nb = std::max<int64_t>(1, std::min<int64_t>(ctas, (Nn + 63) / 64));
+    int64_t nb = std::max<int64_t>(1, std::min<int64_t>(ctas, (Nn + kMinRangeRows - 1) / kMinRangeRows));
     if (p->row_split && nb == p->n_row_split) return FCG_NORMAL_END;
     dfree(p->row_split);
     p->n_row_split = 0;
     int r = dalloc(&p->row_split, nb + 1, p->bytes);
     if (r != FCG_NORMAL_END) return r;
-    k_row_split<<<grid_for(nb + 1, 128, p->ctx->sm_count), 128, 0, p->stream>>>(Nn, p->link_ptr, nb, (double)L + 8.0 * (double)Nn,
+    k_row_split<<<grid_for(nb + 1, 128, p->ctx->sm_count), 128, 0, p->stream>>>(Nn, p->link_ptr, nb, (double)L + kRowWork * (double)Nn,
                                                                                p->row_split);
     FCG_CK(cudaGetLastError());
     p->timings.launches++;
