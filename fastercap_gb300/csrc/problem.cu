@@ -309,7 +309,7 @@ struct DeviceProblem {
     int *active = NULL, *iters = NULL, *capped = NULL, *scap = NULL, *n_active = NULL;
     int *pin = NULL;  // pinned readback slot from the context (NULL: pageable fallback)
     int *pin_dev = NULL;  // the same slot as the device sees it (NULL: no device access)
-    int *d_it = NULL;     // device step state: [0] step index, [1] go on, [2] active solves after the step
+    int *d_it = NULL;     // device step state: [0] step index, [1] go on, [2] active solves after the step, [3] and [4..5] tickets
     double *ptmp = NULL;  // two-level preconditioner output ([k][Np])
     // the Arnoldi loop as one CUDA graph (a while node whose body is one step)
     cudaGraph_t graph = NULL;
@@ -2224,108 +2224,13 @@ __global__ void k_reduce_seg(int nvec, int ks, int G, int nch, const double *__r
     if (lane == 0) out[sidx * ostride_s + j * ostride_j] = sum;
 }
 
-// Givens update of Hessenberg column i of active solve sidx; true while the
-// solve goes on
 // one previous rotation applied to (t1, t2), every product rounded before
-// the sum (no contraction: the per-solve and per-warp Givens kernels round
-// the same way)
+// the sum (no contraction: the chain below forms rot_hi's two products apart)
 __device__ __forceinline__ double rot_lo(double c, double s, double t1, double t2) {
     return __dsub_rn(__dmul_rn(c, t1), __dmul_rn(s, t2));
 }
 __device__ __forceinline__ double rot_hi(double c, double s, double t1, double t2) {
     return __dadd_rn(__dmul_rn(c, t2), __dmul_rn(s, t1));
-}
-
-// the rest of a solve's Givens step once its column's previous rotations
-// are applied (hc[0..i-1] rotated, `carry` the running entry i): the new
-// rotation, the right-hand side, the convergence test
-__device__ bool givens_finish(int sidx, int i, int M, double *hc, double carry, double hn, double *cs, double *sn, double *g,
-                              const double *normb, double tol, const int *scap, int *active, int *iters, int *capped) {
-    double *c = cs + (int64_t)sidx * (M + 2), *sv = sn + (int64_t)sidx * (M + 2), *gg = g + (int64_t)sidx * (M + 2);
-    hc[i] = carry;
-    double t1 = carry, t2 = hn;
-    double len = __dsqrt_rn(__dadd_rn(__dmul_rn(t1, t1), __dmul_rn(t2, t2)));
-    c[i] = t1 / len;
-    sv[i] = -t2 / len;
-    hc[i] = rot_lo(c[i], sv[i], t1, t2);
-    hc[i + 1] = 0;
-    t1 = gg[i];
-    gg[i] = c[i] * t1;
-    gg[i + 1] = sv[i] * t1;
-    double res = fabs(gg[i + 1]) / normb[sidx];
-    if (res < tol) {
-        active[sidx] = 0;
-        iters[sidx] = i;
-    } else if (i + 1 >= scap[sidx]) {
-        // the solve's iteration cap: keep the last Arnoldi step
-        active[sidx] = 0;
-        iters[sidx] = i;
-        capped[sidx] = 1;
-    } else {
-        return true;
-    }
-    return false;
-}
-
-__device__ bool givens_one(int sidx, int i, int M, double *const *__restrict__ Hp, double *cs, double *sn, double *g,
-                           const double *normb, const double *nrm2, double *hnorm, double *rhnorm, double tol, const int *scap,
-                           int *active, int *iters, int *capped) {
-    double *hc = Hp[i] + (int64_t)sidx * (i + 2);
-    const double *c = cs + (int64_t)sidx * (M + 2), *sv = sn + (int64_t)sidx * (M + 2);
-    double hn = sqrt(nrm2[sidx]);
-    hnorm[sidx] = hn;
-    if (rhnorm) rhnorm[sidx] = 1.0 / hn;
-    hc[i + 1] = hn;
-    // the previous rotations, in order; the running entry stays in a register
-    // so the loads of the next column entries and rotations do not wait on it
-    double carry = hc[0];
-#pragma unroll 8
-    for (int j = 0; j < i; j++) {
-        double t1 = carry, t2 = hc[j + 1];
-        hc[j] = rot_lo(c[j], sv[j], t1, t2);
-        carry = rot_hi(c[j], sv[j], t1, t2);
-    }
-    return givens_finish(sidx, i, M, hc, carry, hn, cs, sn, g, normb, tol, scap, active, iters, capped);
-}
-
-// Givens update of Hessenberg column i of every active solve, one warp per solve: the lanes load 32 entries of the
-// column and of the previous rotations at a time, and every lane runs the
-// chain of rotations on shuffled values (the same operations in the same
-// order as k_givens), so a step waits for memory once per 32 rotations.
-__global__ void __launch_bounds__(128) k_givens_warp(int S, const int *__restrict__ iter, int M, double *const *__restrict__ Hp,
-                                                     double *cs, double *sn, double *g, const double *normb, const double *nrm2,
-                                                     double *hnorm, double *rhnorm, double tol, const int *scap, int *active,
-                                                     int *iters, int *capped, int *n_active_all) {
-    const int i = *iter;
-    const int sidx = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (sidx >= S || !active[sidx]) return;  // the whole warp
-    double *hc = Hp[i] + (int64_t)sidx * (i + 2);
-    const double *c = cs + (int64_t)sidx * (M + 2), *sv = sn + (int64_t)sidx * (M + 2);
-    const double hn = sqrt(nrm2[sidx]);
-    double carry = hc[0];
-    for (int j0 = 0; j0 < i; j0 += 32) {
-        const int j = j0 + lane, cnt = min(32, i - j0);
-        double cj = 0.0, sj = 0.0, hj = 0.0, out = 0.0;
-        if (j < i) {
-            cj = c[j];
-            sj = sv[j];
-            hj = hc[j + 1];
-        }
-        for (int q = 0; q < cnt; q++) {
-            const double cq = __shfl_sync(0xffffffffu, cj, q), sq = __shfl_sync(0xffffffffu, sj, q);
-            const double t1 = carry, t2 = __shfl_sync(0xffffffffu, hj, q);
-            const double h = rot_lo(cq, sq, t1, t2);
-            carry = rot_hi(cq, sq, t1, t2);
-            if (lane == q) out = h;
-        }
-        __syncwarp();  // every lane has read the entries it overwrites next
-        if (j < i) hc[j] = out;
-    }
-    if (lane != 0) return;
-    hnorm[sidx] = hn;
-    if (rhnorm) rhnorm[sidx] = 1.0 / hn;
-    if (givens_finish(sidx, i, M, hc, carry, hn, cs, sn, g, normb, tol, scap, active, iters, capped))
-        atomicAdd(n_active_all + i, 1);
 }
 
 // out[r][j] = v[r][j] / hn[solve of (j, r)] for active solves, out = out_fixed
@@ -2390,18 +2295,9 @@ __device__ void iter_advance_one(int *iter, int i, int na, int cap, const volati
     if (use_cond) cudaGraphSetConditional(cond, go ? 1u : 0u);
 }
 
-// end of an Arnoldi step (one thread): advance the step index; go on while
-// a solve is active, the basis has room and no cancellation was asked for.
-// Inside the graph's while loop it sets the loop condition.
-__global__ void k_iter_advance(int *iter, const int *__restrict__ n_active, int cap, const volatile int *cancel, int *state,
-                               cudaGraphConditionalHandle cond, int use_cond) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int i = *iter;
-    iter_advance_one(iter, i, n_active[i], cap, cancel, state, cond, use_cond);
-}
-
-// What ends an Arnoldi step (k_reduce_seg of the norms, k_givens,
-// k_iter_advance) when the last CTA of k_update runs it.
+// What ends an Arnoldi step: every solve's norm and Givens update, then the
+// step index and the loop condition (step_end in k_update's last CTA for a few
+// solves, k_step_end for many).
 struct StepEnd {
     int S, ks, G, M, cap, use_cond;
     const int32_t *g_ch_first, *g_ch_count;
@@ -2415,36 +2311,120 @@ struct StepEnd {
     cudaGraphConditionalHandle cond;
 };
 
-// one CTA: the norm of every active solve (summed over its geometry's
-// chunks in the same order as k_reduce_seg), the Givens update, then the
-// step index and the loop condition
+// One warp: the norm of active solve sidx (summed over its geometry's chunks
+// in the same order as k_reduce_seg) and its Givens update of Hessenberg
+// column i; lane 0 says whether the solve goes on.
+//
+// The previous rotations are a serial chain in FP64, whose pipe takes about
+// 20 cycles an SM for every warp instruction: so the chain is only what is
+// serial in it, carry = c h + s carry, one product and one sum a rotation
+// (the lanes form their c h, and afterwards their rotated entries from the
+// carry that reached them, for 32 rotations at a time), solves take a warp on
+// an SM each, the new rotation's and the norm's quotients are three lanes of
+// one division, and k_step_end's solves meet in one atomic. 53 steps of 22
+// solves: 12.6 + 4.1 + 2.7 us a step as three kernels (norms, Givens on four
+// solves a CTA with six FP64 instructions a rotation, step index), 9.2 us as one
+__device__ bool step_end_warp(const StepEnd &e, int sidx, int i, const double *partial, int nch, double2 *sh) {
+    const int lane = threadIdx.x & 31;
+    double *hc = e.Hp[i] + (int64_t)sidx * (i + 2);
+    const int64_t at = (int64_t)sidx * (e.M + 2);
+    const double *c = e.cs + at, *sv = e.sn + at;
+    const double gi = e.g[at + i], nb = e.normb[sidx];
+    const int cap = e.scap[sidx];
+    double cj = 0.0, sj = 0.0, hj = 0.0;
+    if (lane < i) {
+        cj = c[lane];
+        sj = sv[lane];
+        hj = __ldcg(&hc[lane + 1]);
+    }
+    double carry = __ldcg(&hc[0]);
+    double sum = 0.0;
+    const int r = sidx % e.ks, gg = sidx / e.ks;
+    const int c0 = e.g_ch_first[gg], cn = e.g_ch_count[gg];
+    const double *pp = partial + (int64_t)r * nch + c0;
+#pragma unroll 4
+    for (int k = lane; k < cn; k += 32) sum += __ldcg(&pp[k]);
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    for (int j0 = 0; j0 < i; j0 += 32) {
+        const int j = j0 + lane, cnt = min(32, i - j0);
+        if (j0 > 0 && j < i) {
+            cj = c[j];
+            sj = sv[j];
+            hj = __ldcg(&hc[j + 1]);
+        }
+        sh[lane] = make_double2(__dmul_rn(cj, hj), sj);
+        __syncwarp();  // also: every lane has read the entries overwritten below
+        double mine = 0.0;
+#pragma unroll 8
+        for (int q = 0; q < cnt; q++) {
+            const double2 x = sh[q];
+            if (lane == q) mine = carry;
+            carry = __dadd_rn(x.x, __dmul_rn(x.y, carry));
+        }
+        if (j < i) hc[j] = rot_lo(cj, sj, mine, hj);
+        __syncwarp();
+    }
+    // the new rotation (t1, t2) -> (len, 0) and the right-hand side
+    const double hn = sqrt(sum), t1 = carry, t2 = hn;
+    const double len = __dsqrt_rn(__dadd_rn(__dmul_rn(t1, t1), __dmul_rn(t2, t2)));
+    const double quo = (lane == 0 ? t1 : (lane == 1 ? -t2 : 1.0)) / (lane < 2 ? len : hn);
+    const double ci = __shfl_sync(0xffffffffu, quo, 0), si = __shfl_sync(0xffffffffu, quo, 1), rhn = __shfl_sync(0xffffffffu, quo, 2);
+    if (lane != 0) return false;
+    const double g1 = si * gi, res = fabs(g1) / nb;
+    e.nrm2[sidx] = sum;
+    e.hnorm[sidx] = hn;
+    if (e.rhnorm) e.rhnorm[sidx] = rhn;
+    e.cs[at + i] = ci;
+    e.sn[at + i] = si;
+    hc[i] = rot_lo(ci, si, t1, t2);
+    hc[i + 1] = 0;
+    e.g[at + i] = ci * gi;
+    e.g[at + i + 1] = g1;
+    if (res < e.tol) {
+        e.active[sidx] = 0;
+        e.iters[sidx] = i;
+    } else if (i + 1 >= cap) {
+        // the solve's iteration cap: keep the last Arnoldi step
+        e.active[sidx] = 0;
+        e.iters[sidx] = i;
+        e.capped[sidx] = 1;
+    } else {
+        return true;
+    }
+    return false;
+}
+
+// one CTA of 256 threads ends the step for all (few) solves
 __device__ void step_end(const StepEnd &e, int i, double *partial, int nch) {
     __shared__ int s_na;
-    const int lane = threadIdx.x & 31;
+    __shared__ double2 s_rot[8][32];
+    const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_na = 0;
-    for (int sidx = threadIdx.x >> 5; sidx < e.S; sidx += blockDim.x >> 5) {
-        if (!e.active[sidx]) continue;
-        int r = sidx % e.ks, gg = sidx / e.ks;
-        double sum = 0.0;
-        int c0 = e.g_ch_first[gg], cn = e.g_ch_count[gg];
-        const double *pp = partial + (int64_t)r * nch + c0;
-        for (int c = lane; c < cn; c += 32) sum += __ldcg(&pp[c]);
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) e.nrm2[sidx] = sum;
-    }
     __syncthreads();
-    int na = 0;
-    for (int sidx = threadIdx.x; sidx < e.S; sidx += blockDim.x)
-        if (e.active[sidx] &&
-            givens_one(sidx, i, e.M, e.Hp, e.cs, e.sn, e.g, e.normb, e.nrm2, e.hnorm, e.rhnorm, e.tol, e.scap, e.active, e.iters,
-                       e.capped))
-            na++;
-    if (na) atomicAdd(&s_na, na);
+    for (int sidx = warp; sidx < e.S; sidx += blockDim.x >> 5)
+        if (e.active[sidx] && step_end_warp(e, sidx, i, partial, nch, s_rot[warp])) atomicAdd(&s_na, 1);
     __syncthreads();
     if (threadIdx.x == 0) {
         e.n_active_all[i] = s_na;
         iter_advance_one(e.iter, i, s_na, e.cap, e.cancel, e.state, e.cond, e.use_cond);
     }
+}
+
+// the same for many solves: one warp (one CTA) per solve; the last one to
+// finish (a ticket on *done: solves done, solves that go on in the high word;
+// reset by it) advances the step
+__global__ void __launch_bounds__(32) k_step_end(const StepEnd e, const double *__restrict__ partial, int nch,
+                                                 unsigned long long *done) {
+    __shared__ double2 s_rot[32];
+    const int i = *e.iter, sidx = blockIdx.x;
+    const bool on = e.active[sidx] && step_end_warp(e, sidx, i, partial, nch, s_rot);
+    if (threadIdx.x != 0) return;
+    const unsigned long long mine = 1ull + (on ? 1ull << 32 : 0ull), old = atomicAdd(done, mine);
+    if ((unsigned)old != gridDim.x - 1) return;
+    const int na = (int)((old + mine) >> 32);
+    *done = 0;
+    e.n_active_all[i] = na;
+    iter_advance_one(e.iter, i, na, e.cap, e.cancel, e.state, e.cond, e.use_cond);
 }
 
 // v[r] = w[r] - sum_j h_j V_j[r] with the solve's own h; partial |v|^2 per
@@ -4465,7 +4445,7 @@ static int ensure_solve_ws(DeviceProblem *p, int k, int S, int M) {
             (r = dalloc(&p->x, n, B)))
             return r;
         if ((r = dalloc(&p->Vptr, (size_t)M + 2, B)) || (r = dalloc(&p->Hptr, (size_t)M + 2, B))) return r;
-        if ((r = dalloc(&p->d_it, 4, B))) return r;
+        if ((r = dalloc(&p->d_it, 8, B))) return r;
         p->Vptr_cap = M + 2;
         p->gk = k;
         p->gS = S;
@@ -4733,7 +4713,7 @@ static int enqueue_step(DeviceProblem *p, const StepArgs &a) {
     if (!fuse_h)
         k_reduce_h<<<gh, 256, 0, s>>>(a.k, a.G, a.nch, p->d_it, p->partial, p->g_ch_first, p->g_ch_count, p->active, p->Hptr);
     // v = w - sum h_j q_j; for a few solves its last CTA ends the step
-    // (norms, Givens, index), for many the three kernels do
+    // (norms, Givens, index), for many k_step_end does
     const bool fuse_end = a.S <= 4;
     const volatile int *cancel = p->pin_dev ? p->pin_dev + 4 : NULL;
     double *rhn = p->precision == FCG_PREC_MIXED ? p->hnorm + a.S : NULL;
@@ -4754,13 +4734,8 @@ static int enqueue_step(DeviceProblem *p, const StepArgs &a) {
 #undef FCG_UPDATE
     int launches = 3 + (fuse_h ? 0 : 1);
     if (!fuse_end) {
-        const int g1v = (int)(((int64_t)a.k * a.G * 32 + 255) / 256);
-        k_reduce_seg<<<g1v, 256, 0, s>>>(1, a.k, a.G, a.nch, p->partial, p->g_ch_first, p->g_ch_count, p->active, p->nrm2, 1, 0);
-        k_givens_warp<<<(a.S * 32 + 127) / 128, 128, 0, s>>>(a.S, p->d_it, a.M, p->Hptr, p->cs, p->sn, p->g, p->normb, p->nrm2,
-                                                              p->hnorm, rhn, a.tol,
-                                    p->scap, p->active, p->iters, p->capped, p->n_active);
-        k_iter_advance<<<1, 32, 0, s>>>(p->d_it, p->n_active, a.cap, cancel, p->d_it + 1, a.cond, a.use_cond);
-        launches += 3;
+        k_step_end<<<a.S, 32, 0, s>>>(fe, p->partial, a.nch, reinterpret_cast<unsigned long long *>(p->d_it + 4));
+        launches++;
     }
     if (!fused_scale) {
         // the two-level path normalises here (its preconditioner reads v first);
@@ -4999,7 +4974,7 @@ int problem_solve(DeviceProblem *p, const fcg_solve_options &opt, double *cap, i
             // does any solve need an Arnoldi step? (read below, after the
             // host has prepared the steps while the device works)
             FCG_CK(cudaMemcpyAsync(pin, p->n_active + M + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-            FCG_CK(cudaMemsetAsync(p->d_it, 0, 4 * sizeof(int), s));
+            FCG_CK(cudaMemsetAsync(p->d_it, 0, 8 * sizeof(int), s));
             if (pk == FCG_PRECOND_TWO_LEVEL && !p->ptmp && (r = dalloc(&p->ptmp, (size_t)k * Np, p->bytes))) {
                 status = r;
                 break;
