@@ -238,6 +238,26 @@ FCG_HD double fcg_enfield_numerical(fcg_d3 r, const float *v, fcg_d3 tn, int rul
     return result;
 }
 
+// The source-triangle-only part of the quadratures: a rule's point (px, py) is
+// v0 + px a + (1 - px - py) b, and `fac` = jacobian / (2 area) (1 up to the
+// rounding of the sides, each a float difference of its own vertices). The
+// frame's expressions with the axes multiplied out: the same points and factor
+// up to FP64 rounding.
+struct fcg_quad64 {
+    double v0[3], a[3], b[3], fac;
+};
+
+FCG_HD void fcg_quad64_make(const float *v, fcg_quad64 &q) {
+    const fcg_quad_frame f = fcg_frame(v);
+    const fcg_d3 s1 = fcg_fsub(v + 3, v + 0);
+    q.v0[0] = f.v0.x; q.v0[1] = f.v0.y; q.v0[2] = f.v0.z;
+    q.a[0] = s1.x; q.a[1] = s1.y; q.a[2] = s1.z;
+    q.b[0] = f.x.x * f.vert2d02 + f.y.x * f.vert2d12;
+    q.b[1] = f.x.y * f.vert2d02 + f.y.y * f.vert2d12;
+    q.b[2] = f.x.z * f.vert2d02 + f.y.z * f.vert2d12;
+    q.fac = (f.jacobian / 2.0) / f.area;
+}
+
 // Unit normal pointing to the outer-permittivity side of a dielectric element.
 // Super nodes store an area-weighted, unnormalised normal.
 FCG_HD fcg_d3 fcg_diel_normal(unsigned type, const float *normal) {

@@ -76,6 +76,26 @@ __device__ __forceinline__ float2 d2pair_bits(double d) {
 // pair -> double: x + y rounded once
 __device__ __forceinline__ double pair2d(float2 p) { return __dadd_rn(f2d_bits(p.x), f2d_bits(p.y)); }
 
+// 1 / sqrt(x), x > 0: the FP32 reciprocal square root of x's leading 24 bits
+// (relative error d0 below 2^-21, the truncation and the approximation) as
+// the seed of one step of Householder's third-order iteration,
+// y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2: the error left is 5/2 d0^3 <
+// 2^-61, so only the five operations' rounding shows (below 2 ulp; the
+// square root and division it stands for round twice). Five FP64
+// instructions instead of about thirty; x whose leading part is no normal
+// float takes the library function out of line.
+__device__ __noinline__ double rsqrt64_rare(double x) { return 1.0 / sqrt(x); }
+
+__device__ __forceinline__ double rsqrt64(double x) {
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    if (hi - (898u << 20) >= (252u << 20)) return rsqrt64_rare(x);
+    const float y0 = rsqrtf(__uint_as_float(((hi - (896u << 20)) << 3) | (lo >> 29)));
+    const uint32_t u = __float_as_uint(y0);
+    const double y = __hiloint2double((int)((u >> 3) + (896u << 20)), (int)(u << 29));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
 }  // namespace
 }  // namespace fcg
 
