@@ -1685,16 +1685,6 @@ template <int LPL, int LPW> __device__ __forceinline__ void slot_reduce(KSum &a,
         }
     }
 }
-template <int LPL, int LPW> __device__ __forceinline__ double slot_reduce64(double a, int lane, int li) {
-#pragma unroll
-    for (int o = 1; o < LPW; o <<= 1) {
-        int from = lane + o * LPL;
-        double oa = __shfl_sync(0xffffffffu, a, from < 32 ? from : lane);
-        if ((li & (2 * o - 1)) == 0 && li + o < LPW) a += oa;
-    }
-    return a;
-}
-
 // Four columns of one link or of a group of links (their products summed
 // plainly) into the compensated sums.
 __device__ __forceinline__ void link_add1(KSum *acc, float c, float4 q) {
@@ -1876,37 +1866,97 @@ __global__ void __launch_bounds__(256, K >= 16 ? 4 : (K >= 8 ? 6 : 7))
     }
 }
 
-// FP64 counterpart: K/2 lanes share a link, each lane owns two right-hand sides.
+// FP64 counterpart: a lane owns CL right-hand sides of a link, two for up to
+// ten columns and four from twelve on, so that K/CL lanes share a link with
+// few lanes of a warp idle (at most two up to K = 24).
+//
+// The FP64 pipe takes about 20 cycles an SM for every warp instruction,
+// whatever its active lanes: so a row's slot sums are not added by a shuffle
+// tree on all lanes (CL log2(slots) additions) but through shared memory, one
+// lane per column and part: lane part * K + c adds column c over the slots
+// part, part + G, ..., then the G parts meet by shuffle. Two (CL = 2) or one link
+// per slot and pass at six CTAs an SM (more links in flight at fewer CTAs
+// are slower, four at four CTAs 86 -> 112 us: half of the rows have some 20
+// links). Microseconds a launch, before (two columns a lane, shuffle tree)
+// and after: 3.4M links 6 columns 113 -> 86 (at 8 columns before), 2 columns
+// 100 -> 57, 12 columns 154 -> 132; 9.6M, 8 columns 259 -> 240; 28.5M, 24
+// columns 1742 -> 1460; slab 20M, 16 columns 913 -> 760.
 template <int K>
-__global__ void __launch_bounds__(256) k_spmv64_multi(const int32_t *__restrict__ row_split, const int64_t *__restrict__ ptr,
+__global__ void __launch_bounds__(256, 6) k_spmv64_multi(const int32_t *__restrict__ row_split, const int64_t *__restrict__ ptr,
                                                       const uint32_t *__restrict__ src, const double *__restrict__ coef,
                                                       const double *__restrict__ Q, double *__restrict__ P) {
-    constexpr int LPL = K / 2, LPW = 32 / LPL;
-    int lane = threadIdx.x & 31, li = lane / LPL, ri = lane % LPL;
-    bool slot_ok = li < LPW;
-    const double2 *Q2 = reinterpret_cast<const double2 *>(Q);
-    int r0 = row_split[blockIdx.x], r1 = row_split[blockIdx.x + 1];
-    for (int row = r0 + (threadIdx.x >> 5); row < r1; row += 8) {
-        double a0 = 0.0, a1 = 0.0;
-        int s = (int)ptr[row], e = (int)ptr[row + 1];
-        int l = s + li;
-        if (slot_ok) {
-            for (; l + LPW < e; l += 2 * LPW) {
-                double c0 = __ldcs(&coef[l]), c1 = __ldcs(&coef[l + LPW]);
-                uint32_t j0 = __ldcs(&src[l]) & kSrcMask, j1 = __ldcs(&src[l + LPW]) & kSrcMask;
-                double2 q0 = Q2[(int64_t)j0 * LPL + ri], q1 = Q2[(int64_t)j1 * LPL + ri];
-                a0 += c0 * q0.x; a1 += c0 * q0.y;
-                a0 += c1 * q1.x; a1 += c1 * q1.y;
+    constexpr int CL = K >= 12 ? 4 : 2, LPL = K / CL, LPW = 32 / LPL, U = 4 / CL;
+    constexpr int G = 32 / K < LPW ? 32 / K : LPW;  // parts of a column's slots
+    __shared__ __align__(16) double red[8][LPW * K];
+    const int lane = threadIdx.x & 31, li = lane / LPL, ri = lane % LPL;
+    double *wred = red[threadIdx.x >> 5];
+    const bool slot_ok = li < LPW;
+    const double2 *Q2 = reinterpret_cast<const double2 *>(Q) + ri * (CL / 2);
+    const int r1 = row_split[blockIdx.x + 1];
+    int row = row_split[blockIdx.x] + (threadIdx.x >> 5);
+    if (row >= r1) return;
+    int s = (int)ptr[row], e = (int)ptr[row + 1];
+    while (true) {
+        int ns = 0, ne = 0;  // the warp's next row
+        if (row + 8 < r1) { ns = (int)ptr[row + 8]; ne = (int)ptr[row + 9]; }
+        double acc[CL];
+#pragma unroll
+        for (int r = 0; r < CL; r++) acc[r] = 0.0;
+        // a pass of U links per slot; lanes past the row's end add nothing,
+        // and no instruction of a link that no slot has is issued
+        for (int l0 = s; l0 < e; l0 += U * LPW) {
+            double c[U];
+            uint32_t j[U];
+            double2 q[U][CL / 2];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int l = l0 + u * LPW + li;
+                const bool ok = slot_ok && l < e;
+                c[u] = ok ? __ldcs(&coef[l]) : 0.0;
+                j[u] = ok ? __ldcs(&src[l]) & kSrcMask : 0u;
             }
-            if (l < e) {
-                double c0 = __ldcs(&coef[l]);
-                double2 q0 = Q2[(int64_t)(__ldcs(&src[l]) & kSrcMask) * LPL + ri];
-                a0 += c0 * q0.x; a1 += c0 * q0.y;
-            }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int r = 0; r < CL / 2; r++)
+                    if (slot_ok && l0 + u * LPW + li < e) q[u][r] = Q2[(int64_t)j[u] * (K / 2) + r];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (l0 + u * LPW < e) {  // the same for the whole warp
+                    if (slot_ok && l0 + u * LPW + li < e) {
+#pragma unroll
+                        for (int r = 0; r < CL / 2; r++) {
+                            acc[2 * r] += c[u] * q[u][r].x;
+                            acc[2 * r + 1] += c[u] * q[u][r].y;
+                        }
+                    }
+                }
         }
-        a0 = slot_reduce64<LPL, LPW>(a0, lane, li);
-        a1 = slot_reduce64<LPL, LPW>(a1, lane, li);
-        if (li == 0) reinterpret_cast<double2 *>(P + (int64_t)row * K)[ri] = make_double2(a0, a1);
+        if (slot_ok) {
+#pragma unroll
+            for (int r = 0; r < CL / 2; r++)
+                reinterpret_cast<double2 *>(wred + li * K + ri * CL)[r] = make_double2(acc[2 * r], acc[2 * r + 1]);
+        }
+        __syncwarp();
+        const int col = lane % K, part = lane / K;
+        double sum = 0.0;
+        if (part < G) {
+            sum = wred[part * K + col];
+#pragma unroll
+            for (int q = G; q < LPW; q += G)
+                if (part + q < LPW) sum += wred[(part + q) * K + col];
+        }
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const double other = __shfl_down_sync(0xffffffffu, sum, o * K);
+            if ((part & (2 * o - 1)) == 0 && part + o < G) sum += other;
+        }
+        if (lane < K) P[(int64_t)row * K + lane] = sum;
+        __syncwarp();  // the buffer is reused by the warp's next row
+        row += 8;
+        if (row >= r1) return;
+        s = ns;
+        e = ne;
     }
 }
 
@@ -3945,8 +3995,13 @@ int problem_get_coefficients(DeviceProblem *p, double *link_coef, double *self_c
 }
 
 // node-work columns for k right-hand sides: 1, 2, else a multiple of four
-// (the multi-right-hand-side link product moves four per 16-byte gather)
+// (the mixed multi-right-hand-side link product moves four per 16-byte
+// gather); FP64 up to ten, where a lane owns two columns and every padding
+// column costs its share of the FP64 pipe, an even number
 static int kpad(int k) { return k <= 2 ? k : (k + 3) / 4 * 4; }
+static int kpad(const DeviceProblem *p, int k) {
+    return p->precision == FCG_PREC_FP64 && k <= 10 ? (k == 1 ? 1 : (k + 1) / 2 * 2) : kpad(k);
+}
 
 static int ensure_matvec_ws(DeviceProblem *p, int kp) {
     if (p->kcap >= kp) return FCG_NORMAL_END;
@@ -4022,7 +4077,9 @@ static void launch_link(DeviceProblem *p, const NodeWork &w, int kp, bool mixed)
             switch (kp) {
             case 2: FCG_MULTI64(2); break;
             case 4: FCG_MULTI64(4); break;
+            case 6: FCG_MULTI64(6); break;
             case 8: FCG_MULTI64(8); break;
+            case 10: FCG_MULTI64(10); break;
             case 12: FCG_MULTI64(12); break;
             case 16: FCG_MULTI64(16); break;
             case 20: FCG_MULTI64(20); break;
@@ -4254,11 +4311,11 @@ static int choose_rhs_width(DeviceProblem *p, int cols, int *width) {
         return FCG_DEVICE_ERROR;
     }
     // the workspace for the widest candidate serves them all
-    int r = ensure_matvec_ws(p, kpad(full));
+    int r = ensure_matvec_ws(p, kpad(p, full));
     double best = 1e300;
     int best_w = full;
     for (size_t i = 0; i < cand.size() && r == FCG_NORMAL_END; i++) {
-        int w = cand[i], kp = kpad(w);
+        int w = cand[i], kp = kpad(p, w);
         if ((r = autotune(p, kp)) != FCG_NORMAL_END) break;
         NodeWork nw = {p->Qd, p->Qf, p->Pd, p->Pf2, p->Ad};
         launch_link(p, nw, kp, true);  // warm
@@ -4292,7 +4349,7 @@ static int choose_rhs_width(DeviceProblem *p, int cols, int *width) {
 // v = P * (in / diag) for k right-hand sides ([k][Np] device arrays)
 static int matvec(DeviceProblem *p, const double *in, double *out, int k, const double *diag, const StepScale *scale = NULL) {
     if (k < 1 || k > kMaxK) { set_error("right-hand sides per matvec must be in [1, 32]"); return FCG_GENERIC_ERROR; }
-    int kp = kpad(k);
+    int kp = kpad(p, k);
     int r = ensure_matvec_ws(p, kp);
     if (r == FCG_NORMAL_END) r = autotune(p, kp);
     if (r != FCG_NORMAL_END) return r;
@@ -5049,7 +5106,7 @@ int problem_solve(DeviceProblem *p, const fcg_solve_options &opt, double *cap, i
             }
             StepArgs sa = {k, S, G, M, nch, M, pk, pair_basis ? 1 : 0, chunks, diag, opt.tol, 0, 0};
             // the workspace a step touches exists before any capture
-            if ((r = ensure_matvec_ws(p, kpad(k))) || (r = autotune(p, kpad(k))) ||
+            if ((r = ensure_matvec_ws(p, kpad(p, k))) || (r = autotune(p, kpad(p, k))) ||
                 (pk == FCG_PRECOND_TWO_LEVEL && (r = precond_apply(p, pk, p->vv, p->ptmp, k)))) {
                 status = r;
                 break;
