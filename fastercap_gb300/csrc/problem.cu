@@ -54,7 +54,7 @@ namespace fcg {
 static const int kBlockLeaves = 256;  // leaves per sweep subtree
 static const int kMaxChain = 96;      // ancestors above a sweep subtree
 static const int kSweepCols = 4;      // right-hand sides per shared-memory pass of the sweeps
-static const int kSweepThreads = 128;  // threads per sweep CTA
+static const int kSweepThreads = 128;  // nodes a sweep CTA takes at a time (its threads, or half of them)
 static const int kMaxK = 32;          // right-hand sides per matvec batch
 static const int kDotChunk = 1024;    // vector elements per CTA in the Krylov kernels
 static const int kDotThreads = 128;   // threads per chunk in k_dots
@@ -939,8 +939,11 @@ __global__ void k_fill_self(int64_t Np, const int32_t *__restrict__ leaf_node, c
 // (left + right, in FP64), so a level costs a barrier, not a round trip to
 // memory. Node charges go to Qf (mixed) or Qd (FP64); the mixed path also
 // keeps the block root's FP64 charge for the top pass. Leaf j has device
-// label j. Right-hand sides are processed kc at a time; kSweepThreads
-// threads per CTA keep every block of a large model resident at once.
+// label j. CTA (block, y) takes right-hand sides y kc .. y kc + kc - 1 (a
+// CTA per block that took them one pass after the other left a small model's
+// SMs with one CTA each: 6 columns, 38k panels, 24.7 -> 17.1 us);
+// kSweepThreads threads per CTA keep every block of a large model resident
+// at once.
 // The Arnoldi step's pending normalisation, done by the up-sweep as it reads
 // the step's vector (k_scale's work): q = v / |v| for every active solve,
 // written back to v and to basis vector *iter (FP64, or an FP32 pair on the
@@ -956,7 +959,7 @@ struct StepScale {
 };
 
 template <bool MIXED>
-__global__ void __launch_bounds__(kSweepThreads, 16) k_up_blk(const SweepPlan plan, const double *in, int64_t ld, int k, int kp,
+__global__ void __launch_bounds__(kSweepThreads, 10) k_up_blk(const SweepPlan plan, const double *in, int64_t ld, int k, int kp,
                                                               int kc, const double *__restrict__ diag, int recip,
                                                               double *__restrict__ Qd, float *__restrict__ Qf,
                                                               double *__restrict__ rootq, const StepScale sc) {
@@ -965,7 +968,7 @@ __global__ void __launch_bounds__(kSweepThreads, 16) k_up_blk(const SweepPlan pl
     uint32_t *kids = (uint32_t *)(sh + (2 * kBlockLeaves - 1) * kc);  // kBlockLeaves
     int32_t *lbl = (int32_t *)(kids + kBlockLeaves);                  // kBlockLeaves
     int32_t *lp = lbl + kBlockLeaves;                                 // kBlockLeaves + 1
-    const int b = blockIdx.x, tid = threadIdx.x;
+    const int b = blockIdx.x, tid = threadIdx.x, c0 = blockIdx.y * kc, kk = min(kc, k - c0);
     const int lf = plan.blk_leaf_first[b], nl = plan.blk_nleaves[b], lv0 = plan.blk_lvl_first[b], H = plan.blk_nlvls[b];
     const int base = plan.blk_node_first[b], ni = nl - 1;
     for (int t = tid; t < ni; t += blockDim.x) {
@@ -975,43 +978,38 @@ __global__ void __launch_bounds__(kSweepThreads, 16) k_up_blk(const SweepPlan pl
     for (int t = tid; t <= H; t += blockDim.x) lp[t] = plan.lvl_ptr[lv0 + t] - base;
     const int step = sc.hn ? *sc.iter : 0;
     double *Vi = step > 0 ? sc.Vp[step] : NULL;
-    for (int c0 = 0; c0 < k; c0 += kc) {
-        const int kk = min(kc, k - c0);
-        for (int t = tid; t < nl * kk; t += blockDim.x) {
-            int r = t / nl, i = t - r * nl;
-            int64_t at = (int64_t)(c0 + r) * ld + lf + i;
-            double x = in[at];
-            if (Vi) {
-                int sidx = sc.leaf_geom[lf + i] * k + c0 + r;
-                if (sc.active[sidx]) {
-                    x = sc.recip ? x * sc.hn[sidx] : x / sc.hn[sidx];
-                    const_cast<double *>(in)[at] = x;
-                    if (sc.pair) reinterpret_cast<float2 *>(Vi)[at] = d2pair_bits(x);
-                    else Vi[at] = x;
-                }
-            }
-            if (diag) x = recip ? x * diag[lf + i] : x / diag[lf + i];
-            val[i * kc + r] = x;
-            int64_t o = (int64_t)(lf + i) * kp + c0 + r;
-            if (!MIXED || ni == 0) Qd[o] = x;
-            if (MIXED) Qf[o] = (float)x;
-            if (ni == 0) rootq[(int64_t)b * kp + c0 + r] = x;
+    const int s0 = Vi ? sc.leaf_geom[lf] * k + c0 : 0;  // a block lies in one geometry
+    for (int t = tid; t < nl * kk; t += blockDim.x) {
+        int r = t / nl, i = t - r * nl;
+        int64_t at = (int64_t)(c0 + r) * ld + lf + i;
+        double x = in[at];
+        if (Vi && sc.active[s0 + r]) {
+            x = sc.recip ? x * sc.hn[s0 + r] : x / sc.hn[s0 + r];
+            const_cast<double *>(in)[at] = x;
+            if (sc.pair) reinterpret_cast<float2 *>(Vi)[at] = d2pair_bits(x);
+            else Vi[at] = x;
+        }
+        if (diag) x = recip ? x * diag[lf + i] : x / diag[lf + i];
+        val[i * kc + r] = x;
+        int64_t o = (int64_t)(lf + i) * kp + c0 + r;
+        if (!MIXED || ni == 0) Qd[o] = x;
+        if (MIXED) Qf[o] = (float)x;
+        if (ni == 0) rootq[(int64_t)b * kp + c0 + r] = x;
+    }
+    __syncthreads();
+    for (int h = 0; h < H; h++) {
+        const int a = lp[h], cnt = lp[h + 1] - a;
+        for (int t = tid; t < cnt * kk; t += blockDim.x) {
+            int q = a + t / kk, r = t - (t / kk) * kk;
+            uint32_t kd = kids[q];
+            double sum = val[(kd & 0xffffu) * kc + r] + val[(kd >> 16) * kc + r];
+            val[(nl + q) * kc + r] = sum;
+            int64_t o = (int64_t)lbl[q] * kp + c0 + r;
+            if (!MIXED || q == ni - 1) Qd[o] = sum;  // the root is the block's last (highest) node
+            if (MIXED) Qf[o] = (float)sum;
+            if (q == ni - 1) rootq[(int64_t)b * kp + c0 + r] = sum;
         }
         __syncthreads();
-        for (int h = 0; h < H; h++) {
-            const int a = lp[h], cnt = lp[h + 1] - a;
-            for (int t = tid; t < cnt * kk; t += blockDim.x) {
-                int q = a + t / kk, r = t - (t / kk) * kk;
-                uint32_t kd = kids[q];
-                double sum = val[(kd & 0xffffu) * kc + r] + val[(kd >> 16) * kc + r];
-                val[(nl + q) * kc + r] = sum;
-                int64_t o = (int64_t)lbl[q] * kp + c0 + r;
-                if (!MIXED || q == ni - 1) Qd[o] = sum;  // the root is the block's last (highest) node
-                if (MIXED) Qf[o] = (float)sum;
-                if (q == ni - 1) rootq[(int64_t)b * kp + c0 + r] = sum;
-            }
-            __syncthreads();
-        }
     }
 }
 
@@ -1085,16 +1083,16 @@ __device__ __forceinline__ double pval(const float2 *P, int64_t i) {
 
 // Down-sweep (CMultHier::ComputeLeafPotentials_fast, Solver/MultiplyHierarchical.cpp:231-283):
 // A(n) = P(n) + A(parent(n)) from the top. One CTA per block: the link
-// potentials of the block's nodes and of its root's ancestors, the leaves'
-// scaled inputs and self terms are staged in shared memory (each thread
-// fetches a node's label and then its potential, so the staging is two
-// dependent rounds of loads), the ancestors are summed top down (the
+// potentials of the block's nodes and of its root's ancestors are staged in
+// shared memory (each thread fetches a node's label and then its potential,
+// so the staging is two dependent rounds of loads), the leaves' inputs in
+// registers, the ancestors are summed top down (the
 // reference's order), then every internal node, level by level from the
 // root, adds its A to its internal children's P (which makes their A) or
 // hands it to its leaf children, and every leaf writes
 // v = (self * x + P(leaf)) + A(parent(leaf)).
 template <class TP>
-__global__ void __launch_bounds__(kSweepThreads, 16) k_down_blk(const SweepPlan plan, const double *__restrict__ in, int64_t ld,
+__global__ void __launch_bounds__(kSweepThreads, 10) k_down_blk(const SweepPlan plan, const double *__restrict__ in, int64_t ld,
                                                                 int k, int kp, int kc, const double *__restrict__ diag,
                                                                 int recip, const double *__restrict__ self,
                                                                 const TP *__restrict__ P, double *__restrict__ out) {
@@ -1102,66 +1100,74 @@ __global__ void __launch_bounds__(kSweepThreads, 16) k_down_blk(const SweepPlan 
     double *pv = sh;                                     // (2 kBlockLeaves - 1) x kc: P, then A of internal nodes
     double *al = pv + (2 * kBlockLeaves - 1) * kc;       // kBlockLeaves x kc: A of each leaf's parent
     double *cp = al + kBlockLeaves * kc;                 // kMaxChain x kc: P of the root's ancestors
-    double *ss = cp + kMaxChain * kc;                    // kBlockLeaves: leaf self terms
-    uint32_t *kids = (uint32_t *)(ss + kBlockLeaves);    // kBlockLeaves
+    uint32_t *kids = (uint32_t *)(cp + kMaxChain * kc);  // kBlockLeaves
     int32_t *lp = (int32_t *)(kids + kBlockLeaves);      // kBlockLeaves + 1
-    const int b = blockIdx.x, tid = threadIdx.x;
+    const int b = blockIdx.x, tid = threadIdx.x, c0 = blockIdx.y * kc, kk = min(kc, k - c0);
     const int lf = plan.blk_leaf_first[b], nl = plan.blk_nleaves[b], lv0 = plan.blk_lvl_first[b], H = plan.blk_nlvls[b];
     const int base = plan.blk_node_first[b], ni = nl - 1;
     const int ch0 = plan.blk_chain[b], nc = plan.blk_chain[b + 1] - ch0;
     for (int t = tid; t <= H; t += blockDim.x) lp[t] = plan.lvl_ptr[lv0 + t] - base;
-    for (int t = tid; t < nl; t += blockDim.x) ss[t] = self[lf + t];
+    for (int t = tid; t < ni; t += blockDim.x) {
+        kids[t] = plan.lvl_kids[base + t];
+        int64_t o = (int64_t)plan.lvl_nodes[base + t] * kp + c0;
+        for (int r = 0; r < kk; r++) pv[(nl + t) * kc + r] = pval(P, o + r);
+    }
+    for (int t = tid; t < nc; t += blockDim.x) {
+        int64_t o = (int64_t)plan.chain[ch0 + t] * kp + c0;
+        for (int r = 0; r < kk; r++) cp[t * kc + r] = pval(P, o + r);
+    }
+    for (int t = tid; t < nl * kk; t += blockDim.x) {
+        int i = t / kk, r = t - i * kk;
+        pv[i * kc + r] = pval(P, (int64_t)(lf + i) * kp + c0 + r);
+    }
+    // the leaves' self terms and (scaled) inputs, loaded while the levels run
+    constexpr int NX = 8;  // 256 leaves x 4 columns / 128 threads
+    double xv[NX];
+#pragma unroll
+    for (int u = 0; u < NX; u++) {
+        const int t = tid + u * kSweepThreads;
+        xv[u] = 0.0;
+        if (t < nl * kk) {
+            const int r = t / nl, j = lf + t - r * nl;
+            xv[u] = in[(int64_t)(c0 + r) * ld + j];
+        }
+    }
+    __syncthreads();
+    if (tid < kk && nc > 0) {
+        double acc = cp[(nc - 1) * kc + tid];
+        for (int j = nc - 2; j >= 0; j--) acc = cp[j * kc + tid] + acc;
+        if (ni > 0) pv[(nl + ni - 1) * kc + tid] = pv[(nl + ni - 1) * kc + tid] + acc;  // A of the block root
+        else al[tid] = acc;                                                             // a leaf root's parent sum
+    }
+    __syncthreads();
+    for (int h = H - 1; h >= 0; h--) {
+        const int a = lp[h], cnt = lp[h + 1] - a;
+        for (int t = tid; t < cnt * kk; t += blockDim.x) {
+            int q = a + t / kk, r = t - (t / kk) * kk;
+            double A = pv[(nl + q) * kc + r];
+            uint32_t kd = kids[q];
+            int c1 = kd & 0xffffu, c2 = kd >> 16;
+            if (c1 < nl) al[c1 * kc + r] = A;
+            else pv[c1 * kc + r] = pv[c1 * kc + r] + A;
+            if (c2 < nl) al[c2 * kc + r] = A;
+            else pv[c2 * kc + r] = pv[c2 * kc + r] + A;
+        }
+        __syncthreads();
+    }
     const bool hasA = ni > 0 || nc > 0;
-    for (int c0 = 0; c0 < k; c0 += kc) {
-        const int kk = min(kc, k - c0);
-        for (int t = tid; t < ni; t += blockDim.x) {
-            if (c0 == 0) kids[t] = plan.lvl_kids[base + t];
-            int64_t o = (int64_t)plan.lvl_nodes[base + t] * kp + c0;
-            for (int r = 0; r < kk; r++) pv[(nl + t) * kc + r] = pval(P, o + r);
-        }
-        for (int t = tid; t < nc; t += blockDim.x) {
-            int64_t o = (int64_t)plan.chain[ch0 + t] * kp + c0;
-            for (int r = 0; r < kk; r++) cp[t * kc + r] = pval(P, o + r);
-        }
-        for (int t = tid; t < nl * kk; t += blockDim.x) {
-            int r = t / nl, i = t - r * nl;
-            pv[i * kc + r] = pval(P, (int64_t)(lf + i) * kp + c0 + r);
-        }
-        __syncthreads();
-        if (tid < kk && nc > 0) {
-            double acc = cp[(nc - 1) * kc + tid];
-            for (int j = nc - 2; j >= 0; j--) acc = cp[j * kc + tid] + acc;
-            if (ni > 0) pv[(nl + ni - 1) * kc + tid] = pv[(nl + ni - 1) * kc + tid] + acc;  // A of the block root
-            else al[tid] = acc;                                                             // a leaf root's parent sum
-        }
-        __syncthreads();
-        for (int h = H - 1; h >= 0; h--) {
-            const int a = lp[h], cnt = lp[h + 1] - a;
-            for (int t = tid; t < cnt * kk; t += blockDim.x) {
-                int q = a + t / kk, r = t - (t / kk) * kk;
-                double A = pv[(nl + q) * kc + r];
-                uint32_t kd = kids[q];
-                int c1 = kd & 0xffffu, c2 = kd >> 16;
-                if (c1 < nl) al[c1 * kc + r] = A;
-                else pv[c1 * kc + r] = pv[c1 * kc + r] + A;
-                if (c2 < nl) al[c2 * kc + r] = A;
-                else pv[c2 * kc + r] = pv[c2 * kc + r] + A;
-            }
-            __syncthreads();
-        }
-        for (int t = tid; t < nl * kk; t += blockDim.x) {
-            int r = t / nl, i = t - r * nl;
-            int j = lf + i;
-            // the leaf's (scaled) input, read here once instead of staged
-            double xv = in[(int64_t)(c0 + r) * ld + j];
-            if (diag) xv = recip ? xv * diag[j] : xv / diag[j];
-            double v = ss[i] * xv + pv[i * kc + r];
-            if (hasA) v = v + al[i * kc + r];
-            out[(int64_t)(c0 + r) * ld + j] = v;
-        }
-        __syncthreads();  // the next pass reuses the shared arrays
+#pragma unroll
+    for (int u = 0; u < NX; u++) {
+        const int t = tid + u * kSweepThreads;
+        if (t >= nl * kk) break;
+        const int r = t / nl, i = t - r * nl, j = lf + i;
+        double x = xv[u];
+        if (diag) x = recip ? x * diag[j] : x / diag[j];
+        double v = self[j] * x + pv[i * kc + r];
+        if (hasA) v = v + al[i * kc + r];
+        out[(int64_t)(c0 + r) * ld + j] = v;
     }
 }
+static_assert(kBlockLeaves * kSweepCols == 8 * kSweepThreads, "k_down_blk keeps a block's inputs in eight registers a thread");
 
 // ---- mixed-path sweeps in FP32 pairs
 //
@@ -1247,8 +1253,19 @@ template <int KC> __device__ __forceinline__ void store_leading(float *p, const 
     else p[0] = v[0].x;
 }
 
-// Up-sweep, mixed: k_up_blk with the block's sums in FP32 pairs, one thread
-// per node carrying KC right-hand sides; CTA (block, y) takes columns
+// Right-hand sides a thread of the mixed sweeps carries, and threads of a CTA
+// that takes KC of them: two threads share a node's four columns, so that a
+// warp's global and shared accesses cover whole 32-byte groups (four columns a
+// thread: half of every 16-byte access's sector and bank row was another
+// thread's, and half as many warps hid the latency). Down-sweep, with all of
+// its loads ahead of its first barrier: 24 columns, 161k panels 70 -> 53 us,
+// 20 columns, 264k 112 -> 81, 4 columns, 19k 8.1 -> 5.6; up-sweep, with the
+// normalisation's factors read once a thread, at eight CTAs an SM 43.6 ->
+// 42.8, 59.6 -> 59.2 and 7.2 -> 6.0 (it needs every warp: at five CTAs 52.7).
+__host__ __device__ constexpr int sweep_cols(int KC) { return KC == 4 ? 2 : KC; }
+__host__ __device__ constexpr int sweep_threads(int KC) { return kSweepThreads * (KC / sweep_cols(KC)); }
+
+// Up-sweep, mixed: k_up_blk with the block's sums in FP32 pairs; CTA (block, y) takes columns
 // y*KC .. y*KC+KC-1 of all kp (the padding columns k..kp-1 get zero
 // charges), so the column groups of a block run side by side. A leaf's charge is its input
 // (normalised in FP64 first when the step asks for it) rounded to FP32,
@@ -1256,69 +1273,79 @@ template <int KC> __device__ __forceinline__ void store_leading(float *p, const 
 // (the pair's leading part), the block root's pair to rootq for the top
 // pass.
 template <int KC>
-__global__ void __launch_bounds__(kSweepThreads, 8) k_up_blk32(const SweepPlan plan, const double *in, int64_t ld, int k, int kp,
-                                                                const float *__restrict__ rs, float *__restrict__ Qf,
-                                                                float2 *__restrict__ rootq, const StepScale sc) {
+__global__ void __launch_bounds__(sweep_threads(KC), 8)
+    k_up_blk32(const SweepPlan plan, const double *in, int64_t ld, int k, int kp, const float *__restrict__ rs, float *__restrict__ Qf,
+               float2 *__restrict__ rootq, const StepScale sc) {
+    constexpr int C = sweep_cols(KC), TPN = KC / C;
     extern __shared__ __align__(16) float2 shp[];
     float2 *val = shp;                                                // (2 kBlockLeaves - 1) x KC
     uint32_t *kids = (uint32_t *)(shp + (2 * kBlockLeaves - 1) * KC);  // kBlockLeaves
     int32_t *lbl = (int32_t *)(kids + kBlockLeaves);                  // kBlockLeaves
     int32_t *lp = lbl + kBlockLeaves;                                 // kBlockLeaves + 1
-    const int b = blockIdx.x, tid = threadIdx.x;
+    const int b = blockIdx.x, node = threadIdx.x / TPN, cs = threadIdx.x % TPN * C;
     const int lf = plan.blk_leaf_first[b], nl = plan.blk_nleaves[b], lv0 = plan.blk_lvl_first[b], H = plan.blk_nlvls[b];
     const int base = plan.blk_node_first[b], ni = nl - 1;
-    for (int t = tid; t < ni; t += blockDim.x) {
+    for (int t = threadIdx.x; t < ni; t += blockDim.x) {
         kids[t] = plan.lvl_kids[base + t];
         lbl[t] = plan.lvl_nodes[base + t];
     }
-    for (int t = tid; t <= H; t += blockDim.x) lp[t] = plan.lvl_ptr[lv0 + t] - base;
+    for (int t = threadIdx.x; t <= H; t += blockDim.x) lp[t] = plan.lvl_ptr[lv0 + t] - base;
     const int step = sc.hn ? *sc.iter : 0;
     double *Vi = step > 0 ? sc.Vp[step] : NULL;
-    const int c0 = blockIdx.y * KC;
-    {
-        for (int i = tid; i < nl; i += blockDim.x) {
-            const int j = lf + i;
-            double x[KC];
+    const int c0 = blockIdx.y * KC + cs;  // the thread's first column
+    // the pending normalisation of the block's columns (a block lies in one geometry)
+    bool act[C];
+    double hn[C];
+    if (Vi) {
+        const int g = sc.leaf_geom[lf] * k + c0;
 #pragma unroll
-            for (int r = 0; r < KC; r++) x[r] = c0 + r < k ? in[(int64_t)(c0 + r) * ld + j] : 0.0;
-            if (Vi) {
-                const int g = sc.leaf_geom[j] * k;
+        for (int r = 0; r < C; r++) {
+            act[r] = c0 + r < k && sc.active[g + r];
+            hn[r] = c0 + r < k ? sc.hn[g + r] : 1.0;
+        }
+    }
+#pragma unroll 1
+    for (int i = node; i < nl; i += kSweepThreads) {
+        const int j = lf + i;
+        double x[C];
 #pragma unroll
-                for (int r = 0; r < KC; r++) {
-                    if (c0 + r < k && sc.active[g + c0 + r]) {
-                        x[r] = sc.recip ? x[r] * sc.hn[g + c0 + r] : x[r] / sc.hn[g + c0 + r];
-                        const int64_t at = (int64_t)(c0 + r) * ld + j;
-                        const_cast<double *>(in)[at] = x[r];
-                        if (sc.pair) reinterpret_cast<float2 *>(Vi)[at] = d2pair_bits(x[r]);
-                        else Vi[at] = x[r];
-                    }
+        for (int r = 0; r < C; r++) x[r] = c0 + r < k ? in[(int64_t)(c0 + r) * ld + j] : 0.0;
+        if (Vi) {
+#pragma unroll
+            for (int r = 0; r < C; r++) {
+                if (act[r]) {
+                    x[r] = sc.recip ? x[r] * hn[r] : x[r] / hn[r];
+                    const int64_t at = (int64_t)(c0 + r) * ld + j;
+                    const_cast<double *>(in)[at] = x[r];
+                    if (sc.pair) reinterpret_cast<float2 *>(Vi)[at] = d2pair_bits(x[r]);
+                    else Vi[at] = x[r];
                 }
             }
-            const float sj = rs ? rs[j] : 1.0f;
-            float2 q[KC];
+        }
+        const float sj = rs ? rs[j] : 1.0f;
+        float2 q[C];
 #pragma unroll
-            for (int r = 0; r < KC; r++) q[r] = make_float2(rs ? d2f_bits(x[r]) * sj : d2f_bits(x[r]), 0.0f);
-            store_pairs<KC>(val + i * KC, q);
-            store_leading<KC>(Qf + (int64_t)j * kp + c0, q);
-            if (ni == 0) store_pairs<KC>(rootq + (int64_t)b * kp + c0, q);
+        for (int r = 0; r < C; r++) q[r] = make_float2(rs ? d2f_bits(x[r]) * sj : d2f_bits(x[r]), 0.0f);
+        store_pairs<C>(val + i * KC + cs, q);
+        store_leading<C>(Qf + (int64_t)j * kp + c0, q);
+        if (ni == 0) store_pairs<C>(rootq + (int64_t)b * kp + c0, q);
+    }
+    __syncthreads();
+    for (int h = 0; h < H; h++) {
+        const int a = lp[h], cnt = lp[h + 1] - a;
+        for (int t = node; t < cnt; t += kSweepThreads) {
+            const int q = a + t;
+            const uint32_t kd = kids[q];
+            float2 u[C], w[C];
+            load_pairs<C>(val + (kd & 0xffffu) * KC + cs, u);
+            load_pairs<C>(val + (kd >> 16) * KC + cs, w);
+#pragma unroll
+            for (int r = 0; r < C; r++) u[r] = f2_add(u[r], w[r]);
+            store_pairs<C>(val + (nl + q) * KC + cs, u);
+            store_leading<C>(Qf + (int64_t)lbl[q] * kp + c0, u);
+            if (q == ni - 1) store_pairs<C>(rootq + (int64_t)b * kp + c0, u);  // the root is the block's last (highest) node
         }
         __syncthreads();
-        for (int h = 0; h < H; h++) {
-            const int a = lp[h], cnt = lp[h + 1] - a;
-            for (int t = tid; t < cnt; t += blockDim.x) {
-                const int q = a + t;
-                const uint32_t kd = kids[q];
-                float2 u[KC], w[KC];
-                load_pairs<KC>(val + (kd & 0xffffu) * KC, u);
-                load_pairs<KC>(val + (kd >> 16) * KC, w);
-#pragma unroll
-                for (int r = 0; r < KC; r++) u[r] = f2_add(u[r], w[r]);
-                store_pairs<KC>(val + (nl + q) * KC, u);
-                store_leading<KC>(Qf + (int64_t)lbl[q] * kp + c0, u);
-                if (q == ni - 1) store_pairs<KC>(rootq + (int64_t)b * kp + c0, u);  // the root is the block's last (highest) node
-            }
-            __syncthreads();
-        }
     }
 }
 
@@ -1388,93 +1415,115 @@ __global__ void __launch_bounds__(1024) k_up_top32_global(const SweepPlan plan, 
 }
 
 // Down-sweep, mixed: k_down_blk with the link potentials (the link
-// product's compensated (sum, correction) pairs) propagated in FP32 pairs,
-// one thread per node carrying KC right-hand sides; CTA (block, y) takes
-// columns y*KC .. y*KC+KC-1. Every internal node, level by level from the
+// product's compensated (sum, correction) pairs) propagated in FP32 pairs;
+// CTA (block, y) takes columns y*KC .. y*KC+KC-1. Every internal node, level by level from the
 // root, adds its A to both children's P (an internal child's sum is its A,
 // a leaf's is its potential P(leaf) + A(parent)); every leaf writes
 // v = x * sr + potential in FP64 for its columns below k, sr being the
 // leaf's self term times its Jacobi scale.
 template <int KC>
-__global__ void __launch_bounds__(kSweepThreads, 8) k_down_blk32(const SweepPlan plan, const double *__restrict__ in, int64_t ld,
-                                                                 int k, int kp, const double *__restrict__ sr,
-                                                                 const float2 *__restrict__ P, double *__restrict__ out) {
+__global__ void __launch_bounds__(sweep_threads(KC), KC == 4 ? 5 : 8)
+    k_down_blk32(const SweepPlan plan, const double *__restrict__ in, int64_t ld, int k, int kp, const double *__restrict__ sr,
+                 const float2 *__restrict__ P, double *__restrict__ out) {
+    constexpr int C = sweep_cols(KC), TPN = KC / C;
     extern __shared__ __align__(16) float2 shp[];
     float2 *pv = shp;                                    // (2 kBlockLeaves - 1) x KC: P, then A (potential at leaves)
     float2 *cp = pv + (2 * kBlockLeaves - 1) * KC;       // kMaxChain x KC: P of the root's ancestors
-    double *ss = (double *)(cp + kMaxChain * KC);        // kBlockLeaves: leaf self x scale
-    uint32_t *kids = (uint32_t *)(ss + kBlockLeaves);    // kBlockLeaves
-    int32_t *lbl = (int32_t *)(kids + kBlockLeaves);     // kBlockLeaves: internal node labels
-    int32_t *chl = lbl + kBlockLeaves;                   // kMaxChain: ancestor labels
-    int32_t *lp = chl + kMaxChain;                       // kBlockLeaves + 1
-    const int b = blockIdx.x, tid = threadIdx.x, c0 = blockIdx.y * KC;
+    uint32_t *kids = (uint32_t *)(cp + kMaxChain * KC);  // kBlockLeaves
+    int32_t *lp = (int32_t *)(kids + kBlockLeaves);      // kBlockLeaves + 1
+    const int b = blockIdx.x, node = threadIdx.x / TPN, cs = threadIdx.x % TPN * C, c0 = blockIdx.y * KC + cs;
     const int lf = plan.blk_leaf_first[b], nl = plan.blk_nleaves[b], lv0 = plan.blk_lvl_first[b], H = plan.blk_nlvls[b];
     const int base = plan.blk_node_first[b], ni = nl - 1;
     const int ch0 = plan.blk_chain[b], nc = plan.blk_chain[b + 1] - ch0;
-    for (int t = tid; t < kBlockLeaves; t += blockDim.x) {
+    // everything the block reads is on its way before the first wait: a
+    // thread's internal nodes (label, then potential), leaves and ancestor;
+    // the leaves' inputs and self terms stay in registers until the end
+    constexpr int NT = kBlockLeaves / kSweepThreads;
+    int32_t lab[NT], chl = 0;
+    uint32_t kd0[NT];
+#pragma unroll
+    for (int u = 0; u < NT; u++) {
+        const int t = node + u * kSweepThreads;
+        lab[u] = t < ni ? plan.lvl_nodes[base + t] : 0;
+        kd0[u] = t < ni ? plan.lvl_kids[base + t] : 0u;
+    }
+    if (node < nc) chl = plan.chain[ch0 + node];
+    float2 v[NT][C];
+#pragma unroll
+    for (int u = 0; u < NT; u++) {
+        const int i = node + u * kSweepThreads;
+        if (i < nl) load_pairs<C>(P + (int64_t)(lf + i) * kp + c0, v[u]);
+    }
+    for (int t = threadIdx.x; t <= H; t += blockDim.x) lp[t] = plan.lvl_ptr[lv0 + t] - base;
+#pragma unroll
+    for (int u = 0; u < NT; u++) {
+        const int i = node + u * kSweepThreads;
+        if (i < nl) store_pairs<C>(pv + i * KC + cs, v[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < NT; u++) {
+        const int t = node + u * kSweepThreads;
+        if (t < ni) load_pairs<C>(P + (int64_t)lab[u] * kp + c0, v[u]);
+    }
+    float2 vc[C];
+    if (node < nc) load_pairs<C>(P + (int64_t)chl * kp + c0, vc);
+    double x[NT][C], sj[NT];
+#pragma unroll
+    for (int u = 0; u < NT; u++) {
+        const int i = node + u * kSweepThreads, j = lf + i;
+        sj[u] = i < nl ? sr[j] : 0.0;
+#pragma unroll
+        for (int r = 0; r < C; r++) x[u][r] = i < nl && c0 + r < k ? in[(int64_t)(c0 + r) * ld + j] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < NT; u++) {
+        const int t = node + u * kSweepThreads;
         if (t < ni) {
-            kids[t] = plan.lvl_kids[base + t];
-            lbl[t] = plan.lvl_nodes[base + t];
+            store_pairs<C>(pv + (nl + t) * KC + cs, v[u]);
+            if (cs == 0) kids[t] = kd0[u];
         }
-        if (t < nl) ss[t] = sr[lf + t];
-        if (t < nc) chl[t] = plan.chain[ch0 + t];
     }
-    for (int t = tid; t <= H; t += blockDim.x) lp[t] = plan.lvl_ptr[lv0 + t] - base;
-    // the leaves' link potentials need no label: load them with the labels
-    float2 v[KC];
-    for (int i = tid; i < nl; i += blockDim.x) {
-        load_pairs<KC>(P + (int64_t)(lf + i) * kp + c0, v);
-        store_pairs<KC>(pv + i * KC, v);
-    }
+    if (node < nc) store_pairs<C>(cp + node * KC + cs, vc);
     __syncthreads();
-    for (int t = tid; t < ni; t += blockDim.x) {
-        load_pairs<KC>(P + (int64_t)lbl[t] * kp + c0, v);
-        store_pairs<KC>(pv + (nl + t) * KC, v);
-    }
-    for (int t = tid; t < nc; t += blockDim.x) {
-        load_pairs<KC>(P + (int64_t)chl[t] * kp + c0, v);
-        store_pairs<KC>(cp + t * KC, v);
-    }
-    __syncthreads();
-    if (tid < KC && nc > 0) {
-        float2 acc = cp[(nc - 1) * KC + tid];
-        for (int j = nc - 2; j >= 0; j--) acc = f2_add(cp[j * KC + tid], acc);
+    if (threadIdx.x < KC && nc > 0) {
+        const int r = threadIdx.x;
+        float2 acc = cp[(nc - 1) * KC + r];
+        for (int j = nc - 2; j >= 0; j--) acc = f2_add(cp[j * KC + r], acc);
         // A of the block root (P(leaf) + A(parent) for a single-leaf block)
-        pv[(nl + ni - 1) * KC + tid] = f2_add(pv[(nl + ni - 1) * KC + tid], acc);
+        pv[(nl + ni - 1) * KC + r] = f2_add(pv[(nl + ni - 1) * KC + r], acc);
     }
     __syncthreads();
     for (int h = H - 1; h >= 0; h--) {
         const int a = lp[h], cnt = lp[h + 1] - a;
-        for (int t = tid; t < cnt; t += blockDim.x) {
+        for (int t = node; t < cnt; t += kSweepThreads) {
             const int q = a + t;
-            float2 A[KC], u[KC];
-            load_pairs<KC>(pv + (nl + q) * KC, A);
+            float2 A[C], u[C];
+            load_pairs<C>(pv + (nl + q) * KC + cs, A);
             const uint32_t kd = kids[q];
-            const int c1 = kd & 0xffffu, c2 = kd >> 16;
-            load_pairs<KC>(pv + c1 * KC, u);
+            const int c1 = (kd & 0xffffu) * KC + cs, c2 = (kd >> 16) * KC + cs;
+            load_pairs<C>(pv + c1, u);
 #pragma unroll
-            for (int r = 0; r < KC; r++) u[r] = f2_add(u[r], A[r]);
-            store_pairs<KC>(pv + c1 * KC, u);
-            load_pairs<KC>(pv + c2 * KC, u);
+            for (int r = 0; r < C; r++) u[r] = f2_add(u[r], A[r]);
+            store_pairs<C>(pv + c1, u);
+            load_pairs<C>(pv + c2, u);
 #pragma unroll
-            for (int r = 0; r < KC; r++) u[r] = f2_add(u[r], A[r]);
-            store_pairs<KC>(pv + c2 * KC, u);
+            for (int r = 0; r < C; r++) u[r] = f2_add(u[r], A[r]);
+            store_pairs<C>(pv + c2, u);
         }
         __syncthreads();
     }
-    for (int i = tid; i < nl; i += blockDim.x) {
-        const int j = lf + i;
-        double x[KC];
 #pragma unroll
-        for (int r = 0; r < KC; r++) x[r] = c0 + r < k ? in[(int64_t)(c0 + r) * ld + j] : 0.0;
-        float2 pt[KC];
-        load_pairs<KC>(pv + i * KC, pt);
-        const double sj = ss[i];
+    for (int u = 0; u < NT; u++) {
+        const int i = node + u * kSweepThreads, j = lf + i;
+        if (i >= nl) break;
+        float2 pt[C];
+        load_pairs<C>(pv + i * KC + cs, pt);
 #pragma unroll
-        for (int r = 0; r < KC; r++)
-            if (c0 + r < k) out[(int64_t)(c0 + r) * ld + j] = fma(x[r], sj, f2d_bits(pt[r].x)) + f2d_bits(pt[r].y);
+        for (int r = 0; r < C; r++)
+            if (c0 + r < k) out[(int64_t)(c0 + r) * ld + j] = fma(x[u][r], sj[u], f2d_bits(pt[r].x)) + f2d_bits(pt[r].y);
     }
 }
+static_assert(kMaxChain <= kSweepThreads && kBlockLeaves % kSweepThreads == 0, "k_down_blk32 loads one ancestor a thread");
 
 // Link product, FP64 (CMultHier::ComputePanelPotentials_2fast,
 // Solver/MultiplyHierarchical.cpp:141-226): SW lanes per destination node
@@ -4106,8 +4155,9 @@ static int launch_matvec(DeviceProblem *p, const NodeWork &w, const double *in, 
     size_t n = (size_t)p->Nn * kp;
     const int kc = std::min(k, kSweepCols);
     const size_t up_smem = (size_t)(2 * kBlockLeaves - 1) * kc * sizeof(double) + (3 * kBlockLeaves + 1) * sizeof(int32_t);
-    const size_t down_smem = ((size_t)(3 * kBlockLeaves - 1 + kMaxChain) * kc + kBlockLeaves) * sizeof(double) +
+    const size_t down_smem = (size_t)(3 * kBlockLeaves - 1 + kMaxChain) * kc * sizeof(double) +
                              (2 * kBlockLeaves + 1) * sizeof(int32_t);
+    const dim3 sgrid(pl.n_blocks, (k + kc - 1) / kc);  // the FP64 sweeps: blocks x groups of kc columns
     // the mixed path's Jacobi scaling multiplies by the reciprocals (the
     // FP64 path divides, as the reference does)
     const int recip = mixed && diag == p->self && p->rself ? 1 : 0;
@@ -4118,15 +4168,15 @@ static int launch_matvec(DeviceProblem *p, const NodeWork &w, const double *in, 
         // KC right-hand sides per thread and pass (over all kp columns)
         const int KC = kp >= 4 ? 4 : kp;
         const size_t up32 = (size_t)(2 * kBlockLeaves - 1) * KC * sizeof(float2) + (3 * kBlockLeaves + 1) * sizeof(int32_t);
-        const size_t down32 = (size_t)(2 * kBlockLeaves - 1 + kMaxChain) * KC * sizeof(float2) + kBlockLeaves * sizeof(double) +
-                              (3 * kBlockLeaves + kMaxChain + 1) * sizeof(int32_t);
+        const size_t down32 = (size_t)(2 * kBlockLeaves - 1 + kMaxChain) * KC * sizeof(float2) +
+                              (2 * kBlockLeaves + 1) * sizeof(int32_t);
         const dim3 bgrid(pl.n_blocks, kp / KC);
         float2 *rootq = reinterpret_cast<float2 *>(w.Ad);
         const float *rs = recip ? p->rself32 : NULL;
         const double *sr = recip ? p->srself : p->self;
-        if (KC == 4) k_up_blk32<4><<<bgrid, kSweepThreads, up32, s>>>(pl, in, Np, k, kp, rs, w.Qf, rootq, sc);
-        else if (KC == 2) k_up_blk32<2><<<bgrid, kSweepThreads, up32, s>>>(pl, in, Np, k, kp, rs, w.Qf, rootq, sc);
-        else k_up_blk32<1><<<bgrid, kSweepThreads, up32, s>>>(pl, in, Np, k, kp, rs, w.Qf, rootq, sc);
+        if (KC == 4) k_up_blk32<4><<<bgrid, sweep_threads(4), up32, s>>>(pl, in, Np, k, kp, rs, w.Qf, rootq, sc);
+        else if (KC == 2) k_up_blk32<2><<<bgrid, sweep_threads(2), up32, s>>>(pl, in, Np, k, kp, rs, w.Qf, rootq, sc);
+        else k_up_blk32<1><<<bgrid, sweep_threads(1), up32, s>>>(pl, in, Np, k, kp, rs, w.Qf, rootq, sc);
         FCG_CK(cudaGetLastError());
         int64_t launches = 2;
         if (pl.n_top > 0) {
@@ -4153,17 +4203,17 @@ static int launch_matvec(DeviceProblem *p, const NodeWork &w, const double *in, 
         } else {
             FCG_CK(cudaMemsetAsync(w.Pf2, 0, n * sizeof(float2), s));
         }
-        if (KC == 4) k_down_blk32<4><<<bgrid, kSweepThreads, down32, s>>>(pl, in, Np, k, kp, sr, w.Pf2, out);
-        else if (KC == 2) k_down_blk32<2><<<bgrid, kSweepThreads, down32, s>>>(pl, in, Np, k, kp, sr, w.Pf2, out);
-        else k_down_blk32<1><<<bgrid, kSweepThreads, down32, s>>>(pl, in, Np, k, kp, sr, w.Pf2, out);
+        if (KC == 4) k_down_blk32<4><<<bgrid, sweep_threads(4), down32, s>>>(pl, in, Np, k, kp, sr, w.Pf2, out);
+        else if (KC == 2) k_down_blk32<2><<<bgrid, sweep_threads(2), down32, s>>>(pl, in, Np, k, kp, sr, w.Pf2, out);
+        else k_down_blk32<1><<<bgrid, sweep_threads(1), down32, s>>>(pl, in, Np, k, kp, sr, w.Pf2, out);
         FCG_CK(cudaGetLastError());
         p->timings.matvecs++;
         p->timings.launches += launches;
         return FCG_NORMAL_END;
     }
     // w.Ad (n_nodes x kp) holds the block roots' charges in block order
-    if (mixed) k_up_blk<true><<<pl.n_blocks, kSweepThreads, up_smem, s>>>(pl, in, Np, k, kp, kc, dg, recip, w.Qd, w.Qf, w.Ad, sc);
-    else k_up_blk<false><<<pl.n_blocks, kSweepThreads, up_smem, s>>>(pl, in, Np, k, kp, kc, dg, recip, w.Qd, w.Qf, w.Ad, sc);
+    if (mixed) k_up_blk<true><<<sgrid, kSweepThreads, up_smem, s>>>(pl, in, Np, k, kp, kc, dg, recip, w.Qd, w.Qf, w.Ad, sc);
+    else k_up_blk<false><<<sgrid, kSweepThreads, up_smem, s>>>(pl, in, Np, k, kp, kc, dg, recip, w.Qd, w.Qf, w.Ad, sc);
     FCG_CK(cudaGetLastError());
     int64_t launches = 2;
     if (pl.n_top > 0) {
@@ -4198,8 +4248,8 @@ static int launch_matvec(DeviceProblem *p, const NodeWork &w, const double *in, 
         if (mixed) FCG_CK(cudaMemsetAsync(w.Pf2, 0, n * sizeof(float2), s));
         else FCG_CK(cudaMemsetAsync(w.Pd, 0, n * sizeof(double), s));
     }
-    if (mixed) k_down_blk<float2><<<pl.n_blocks, kSweepThreads, down_smem, s>>>(pl, in, Np, k, kp, kc, dg, recip, p->self, w.Pf2, out);
-    else k_down_blk<double><<<pl.n_blocks, kSweepThreads, down_smem, s>>>(pl, in, Np, k, kp, kc, dg, recip, p->self, w.Pd, out);
+    if (mixed) k_down_blk<float2><<<sgrid, kSweepThreads, down_smem, s>>>(pl, in, Np, k, kp, kc, dg, recip, p->self, w.Pf2, out);
+    else k_down_blk<double><<<sgrid, kSweepThreads, down_smem, s>>>(pl, in, Np, k, kp, kc, dg, recip, p->self, w.Pd, out);
     FCG_CK(cudaGetLastError());
     p->timings.matvecs++;
     p->timings.launches += launches;
