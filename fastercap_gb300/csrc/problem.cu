@@ -58,6 +58,7 @@ static const int kSweepThreads = 128;  // nodes a sweep CTA takes at a time (its
 static const int kMaxK = 32;          // right-hand sides per matvec batch
 static const int kDotChunk = 1024;    // vector elements per CTA in the Krylov kernels
 static const int kDotThreads = 128;   // threads per chunk in k_dots
+static const int kUpdatePanel = 64;   // basis vectors k_update holds the addresses of at a time
 static const int kPinSlots = 1024;    // pinned readback slots per context
 static const int kPinSlotInts = 16;
 // link words: source node in the low 29 bits, distance band (0..4) in the top 3
@@ -2280,7 +2281,10 @@ __global__ void __launch_bounds__(kDotThreads) k_dots(int64_t Np, const int *__r
                                                       int *done) {
     using E = typename std::conditional<PB, float2, double>::type;
     constexpr int NW = kDotThreads / 32, U = kDotChunk / kDotThreads;
-    __shared__ E sh[NW][8];
+    // groups of T vectors whose warps' sums wait for one barrier (one per group
+    // held every warp's loads back: 53 steps of 22 columns 141.1 -> 137.8 us)
+    constexpr int NG = 8;
+    __shared__ E sh[NG][NW][8];
     __shared__ int s_last;
     const int T = 8;
     const int nvec = *iter + 1;
@@ -2301,56 +2305,63 @@ __global__ void __launch_bounds__(kDotThreads) k_dots(int64_t Np, const int *__r
         else wv[u] = x;
     }
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int j0 = z * T; j0 < nvec; j0 += Z * T) {
-        E acc[T];
+    for (int p0 = z * T; p0 < nvec; p0 += NG * Z * T) {
+        for (int g = 0; g < NG; g++) {
+            const int j0 = p0 + g * Z * T;
+            if (j0 >= nvec) break;
+            E acc[T];
 #pragma unroll
-        for (int t = 0; t < T; t++) {
-            acc[t] = kv_zero<E>();
-            if (j0 + t < nvec) {
-                const E *v = reinterpret_cast<const E *>(Vp[j0 + t]) + (int64_t)r * Np + base;
+            for (int t = 0; t < T; t++) {
+                acc[t] = kv_zero<E>();
+                if (j0 + t < nvec) {
+                    const E *v = reinterpret_cast<const E *>(Vp[j0 + t]) + (int64_t)r * Np + base;
 #pragma unroll
-                for (int u = 0; u < U; u++) {
-                    int o = threadIdx.x + u * kDotThreads;
-                    if constexpr (PB) {
-                        if (o < len) acc[t] = f2_fma(acc[t], v[o], wv[u]);
-                    } else {
-                        if (o < len) acc[t] += v[o] * wv[u];
+                    for (int u = 0; u < U; u++) {
+                        int o = threadIdx.x + u * kDotThreads;
+                        if constexpr (PB) {
+                            if (o < len) acc[t] = f2_fma(acc[t], v[o], wv[u]);
+                        } else {
+                            if (o < len) acc[t] += v[o] * wv[u];
+                        }
                     }
                 }
             }
-        }
-        // reduce the eight sums over the warp by halving: each step keeps
-        // half of the values and adds the partner lane's copy of them
-        // (4 + 2 + 1 exchanges), then the last value over lane pairs: lane l
-        // ends with vector 4*bit4 + 2*bit3 + bit2 of its index
+            // reduce the eight sums over the warp by halving: each step keeps
+            // half of the values and adds the partner lane's copy of them
+            // (4 + 2 + 1 exchanges), then the last value over lane pairs: lane l
+            // ends with vector 4*bit4 + 2*bit3 + bit2 of its index
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            bool hi = lane & 16;
-            E send = hi ? acc[q] : acc[q + 4];
-            E keep = hi ? acc[q + 4] : acc[q];
-            acc[q] = kv_add(keep, kv_shfl_xor(send, 16));
-        }
+            for (int q = 0; q < 4; q++) {
+                bool hi = lane & 16;
+                E send = hi ? acc[q] : acc[q + 4];
+                E keep = hi ? acc[q + 4] : acc[q];
+                acc[q] = kv_add(keep, kv_shfl_xor(send, 16));
+            }
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-            bool hi = lane & 8;
-            E send = hi ? acc[q] : acc[q + 2];
-            E keep = hi ? acc[q + 2] : acc[q];
-            acc[q] = kv_add(keep, kv_shfl_xor(send, 8));
+            for (int q = 0; q < 2; q++) {
+                bool hi = lane & 8;
+                E send = hi ? acc[q] : acc[q + 2];
+                E keep = hi ? acc[q + 2] : acc[q];
+                acc[q] = kv_add(keep, kv_shfl_xor(send, 8));
+            }
+            {
+                bool hi = lane & 4;
+                E send = hi ? acc[0] : acc[1];
+                E keep = hi ? acc[1] : acc[0];
+                acc[0] = kv_add(keep, kv_shfl_xor(send, 4));
+            }
+            acc[0] = kv_add(acc[0], kv_shfl_xor(acc[0], 2));
+            acc[0] = kv_add(acc[0], kv_shfl_xor(acc[0], 1));
+            if ((lane & 3) == 0) sh[g][warp][((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = acc[0];
         }
-        {
-            bool hi = lane & 4;
-            E send = hi ? acc[0] : acc[1];
-            E keep = hi ? acc[1] : acc[0];
-            acc[0] = kv_add(keep, kv_shfl_xor(send, 4));
-        }
-        acc[0] = kv_add(acc[0], kv_shfl_xor(acc[0], 2));
-        acc[0] = kv_add(acc[0], kv_shfl_xor(acc[0], 1));
-        if ((lane & 3) == 0) sh[warp][((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = acc[0];
         __syncthreads();
-        if (threadIdx.x < T && j0 + threadIdx.x < nvec) {
-            E sum = kv_zero<E>();
-            for (int ww = 0; ww < NW; ww++) sum = kv_add(sum, sh[ww][threadIdx.x]);
-            partial[((int64_t)r * nvec + j0 + threadIdx.x) * ch.n + c] = kv_double(sum);
+        if (threadIdx.x < NG * T) {
+            const int g = threadIdx.x / T, t = threadIdx.x % T, j = p0 + g * Z * T + t;
+            if (j < nvec) {
+                E sum = kv_zero<E>();
+                for (int ww = 0; ww < NW; ww++) sum = kv_add(sum, sh[g][ww][t]);
+                partial[((int64_t)r * nvec + j) * ch.n + c] = kv_double(sum);
+            }
         }
         __syncthreads();
     }
@@ -2598,72 +2609,106 @@ __global__ void __launch_bounds__(32) k_step_end(const StepEnd e, const double *
 // ends the Arnoldi step (step_end: norms, Givens, step index) and resets *done.
 // PB (the mixed path): basis vectors are FP32 pairs and each element's
 // subtraction chain runs in pair arithmetic (w and every h_j split into
-// pairs, f2_fma), rounded to FP64 once for v and its norm. QV basis vectors
-// are loaded per pass: 8 for small models (few CTAs, so the passes' memory
-// waits are the time), else 4; the subtractions are the same either way.
-template <bool PB, int QV>
-__global__ void __launch_bounds__(256, QV == 8 ? 2 : (PB ? 4 : 1)) k_update(int64_t Np, const int *__restrict__ iter, double *const *__restrict__ Vp, const double *__restrict__ w,
-                         double *const *__restrict__ Hp, SegChunks ch, int ks, const int *__restrict__ active,
-                         double *__restrict__ v, double *__restrict__ partial, int fuse_end, StepEnd fe, int *done) {
+// pairs, f2_fma), rounded to FP64 once for v and its norm. The addresses of up
+// to kUpdatePanel basis vectors and their coefficients (split and negated
+// once a CTA, not by every thread) come into shared memory in one round, so a
+// pass over four vectors waits for memory once and not for the address
+// first. Average of a solve's steps, us a launch: 22 columns, 161k panels 134.4
+// -> 130.1 (0.92 of the copy bandwidth), 14 columns, 90k panels 54.9 -> 50.9,
+// 16 columns, 56k 36.8 -> 33.8, 4 columns, 19k (with the step's end) 22.2 ->
+// 13.7. Slower: one or two elements a thread on 1024 or 512 threads, eight or
+// sixteen vectors a pass (fewer warps), and no faster: columns in the reverse
+// of k_dots' order to find its last ones in L2 (127 to 130).
+template <bool PB>
+__global__ void __launch_bounds__(256, PB ? 4 : 2)
+    k_update(int64_t Np, const int *__restrict__ iter, double *const *__restrict__ Vp, const double *__restrict__ w,
+             double *const *__restrict__ Hp, SegChunks ch, int ks, const int *__restrict__ active, double *__restrict__ v,
+             double *__restrict__ partial, int fuse_end, StepEnd fe, int *done) {
     using E = typename std::conditional<PB, float2, double>::type;
+    constexpr int NT = 256, EL = kDotChunk / NT, QV = 4;
     __shared__ double sh[32];
     __shared__ int s_last;
-    const int nvec = *iter + 1;
-    int r = blockIdx.y, c = blockIdx.x;
-    int sidx = ch.geom[c] * ks + r;
+    __shared__ E s_h[kUpdatePanel];
+    __shared__ const E *s_v[kUpdatePanel];
+    const int nvec = *iter + 1, tid = threadIdx.x;
+    const int r = blockIdx.y, c = blockIdx.x;
+    const int sidx = ch.geom[c] * ks + r;
     if (active[sidx]) {
-    const double *h = Hp[nvec - 1] + (int64_t)sidx * (nvec + 1);
-    int64_t base = ch.start[c];
-    int len = ch.len[c];
-    // four elements per thread, each its own subtraction chain (in basis
-    // order); the elements of four basis vectors are loaded before any of
-    // them is used, so one pass waits for memory once per four vectors
-    const int U = kDotChunk / 256;
-    E x[U];
-    int64_t t0 = (int64_t)r * Np + base + threadIdx.x;
+        const double *h = Hp[nvec - 1] + (int64_t)sidx * (nvec + 1);
+        const int len = ch.len[c];
+        const int64_t t0 = (int64_t)r * Np + ch.start[c];
+        E x[EL];
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-        const double wd = (threadIdx.x + u * 256 < len) ? w[t0 + u * 256] : 0.0;
-        if constexpr (PB) x[u] = d2pair_bits(wd);
-        else x[u] = wd;
-    }
-    for (int j0 = 0; j0 < nvec; j0 += QV) {
-        E hv[QV], vv[QV][U];
-#pragma unroll
-        for (int q = 0; q < QV; q++) {
-            const bool okq = j0 + q < nvec;
-            const double hq = okq ? h[j0 + q] : 0.0;
-            if constexpr (PB) {
-                const float2 hp = d2pair_bits(hq);
-                hv[q] = make_float2(-hp.x, -hp.y);
-            } else {
-                hv[q] = hq;
+        for (int u = 0; u < EL; u++) {
+            const double wd = tid + u * NT < len ? w[t0 + tid + u * NT] : 0.0;
+            if constexpr (PB) x[u] = d2pair_bits(wd);
+            else x[u] = wd;
+        }
+        for (int p0 = 0; p0 < nvec; p0 += kUpdatePanel) {
+            const int np = min(kUpdatePanel, nvec - p0);
+            if (p0) __syncthreads();  // the last panel has been read
+            for (int t = tid; t < np; t += NT) {
+                s_v[t] = reinterpret_cast<const E *>(Vp[p0 + t]) + t0;
+                const double hq = h[p0 + t];
+                if constexpr (PB) {
+                    const float2 hp = d2pair_bits(hq);
+                    s_h[t] = make_float2(-hp.x, -hp.y);
+                } else {
+                    s_h[t] = hq;
+                }
             }
-            const E *vj = okq ? reinterpret_cast<const E *>(Vp[j0 + q]) + t0 : NULL;
+            __syncthreads();
+            int j = 0;
+            for (; j + QV <= np; j += QV) {
+                E vv[QV][EL];
 #pragma unroll
-            for (int u = 0; u < U; u++) vv[q][u] = (okq && threadIdx.x + u * 256 < len) ? vj[u * 256] : kv_zero<E>();
-        }
+                for (int q = 0; q < QV; q++) {
+                    const E *vj = s_v[j + q] + tid;
 #pragma unroll
-        for (int q = 0; q < QV; q++)
-            if (j0 + q < nvec)
+                    for (int u = 0; u < EL; u++) vv[q][u] = tid + u * NT < len ? vj[u * NT] : kv_zero<E>();
+                }
 #pragma unroll
-                for (int u = 0; u < U; u++)
-                    if (threadIdx.x + u * 256 < len) {
-                        if constexpr (PB) x[u] = f2_fma(x[u], hv[q], vv[q][u]);
-                        else x[u] = x[u] - hv[q] * vv[q][u];
+                for (int q = 0; q < QV; q++) {
+                    const E hj = s_h[j + q];
+#pragma unroll
+                    for (int u = 0; u < EL; u++) {
+                        if constexpr (PB) x[u] = f2_fma(x[u], hj, vv[q][u]);
+                        else x[u] = x[u] - hj * vv[q][u];
                     }
-    }
-    double s2 = 0.0;
+                }
+            }
+            if (j < np) {  // the rest of the panel, loaded at once too
+                E vv[QV][EL];
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-        if (threadIdx.x + u * 256 < len) {
-            const double xd = kv_double(x[u]);
-            v[t0 + u * 256] = xd;
-            s2 += xd * xd;
+                for (int q = 0; q < QV; q++) {
+                    const bool okq = j + q < np;
+                    const E *vj = okq ? s_v[j + q] + tid : NULL;
+#pragma unroll
+                    for (int u = 0; u < EL; u++) vv[q][u] = okq && tid + u * NT < len ? vj[u * NT] : kv_zero<E>();
+                }
+#pragma unroll
+                for (int q = 0; q < QV; q++) {
+                    if (j + q >= np) break;
+                    const E hj = s_h[j + q];
+#pragma unroll
+                    for (int u = 0; u < EL; u++) {
+                        if constexpr (PB) x[u] = f2_fma(x[u], hj, vv[q][u]);
+                        else x[u] = x[u] - hj * vv[q][u];
+                    }
+                }
+            }
         }
-    }
-    s2 = block_sum(s2, sh);
-    if (threadIdx.x == 0) partial[(int64_t)r * ch.n + c] = s2;
+        double s2 = 0.0;
+#pragma unroll
+        for (int u = 0; u < EL; u++) {
+            if (tid + u * NT < len) {
+                const double xd = kv_double(x[u]);
+                v[t0 + tid + u * NT] = xd;
+                s2 += xd * xd;
+            }
+        }
+        s2 = block_sum(s2, sh);
+        if (tid == 0) partial[(int64_t)r * ch.n + c] = s2;
     }
     if (!fuse_end) return;
     if (threadIdx.x == 0) {
@@ -2676,7 +2721,6 @@ __global__ void __launch_bounds__(256, QV == 8 ? 2 : (PB ? 4 : 1)) k_update(int6
     step_end(fe, nvec - 1, partial, ch.n);
     if (threadIdx.x == 0) *done = 0;
 }
-
 
 // solves whose true residual |b - A x| / |b| is at or above tol
 __global__ void k_refine_count(int S, const double *__restrict__ nr2, const double *__restrict__ nb2, double tol, int *count) {
@@ -4896,16 +4940,11 @@ static int enqueue_step(DeviceProblem *p, const StepArgs &a) {
                   p->hnorm, rhn, p->normb, a.tol, p->scap, p->active, p->iters, p->capped, p->n_active, p->d_it, p->d_it + 1,
                   cancel, a.cond};
     const dim3 ugrid(a.nch, a.k);
-#define FCG_UPDATE(PBV, QV) \
-    k_update<PBV, QV><<<ugrid, 256, 0, s>>>(Np, p->d_it, p->Vptr, p->w, p->Hptr, a.ch, a.k, p->active, p->vv, p->partial, \
-                                            fuse_end ? 1 : 0, fe, p->d_it + 3)
-    if (pair_basis) {
-        if (small) FCG_UPDATE(true, 8);
-        else FCG_UPDATE(true, 4);
-    } else {
-        if (small) FCG_UPDATE(false, 8);
-        else FCG_UPDATE(false, 4);
-    }
+#define FCG_UPDATE(PBV) \
+    k_update<PBV><<<ugrid, 256, 0, s>>>(Np, p->d_it, p->Vptr, p->w, p->Hptr, a.ch, a.k, p->active, p->vv, p->partial, \
+                                        fuse_end ? 1 : 0, fe, p->d_it + 3)
+    if (pair_basis) FCG_UPDATE(true);
+    else FCG_UPDATE(false);
 #undef FCG_UPDATE
     int launches = 3 + (fuse_h ? 0 : 1);
     if (!fuse_end) {
