@@ -7,13 +7,13 @@
 // element for the self interactions, in the host traversal's order) starts a
 // binary recursion tree: a pair either links (a leaf of the recursion tree)
 // or is replaced by two pairs, the children of one side. The frontier is
-// expanded one level per step; the two children of a split pair are placed
-// next to each other, in the order of their parents, so each level keeps the
-// left-to-right order of the recursion trees. A bottom-up pass counts the
-// links under every frontier item and a top-down pass hands out depth-first
+// expanded one level per launch; the two children of a split pair are placed
+// next to each other, wherever in the next level the warp's atomic puts them,
+// and every split pair remembers where. A bottom-up pass counts the links
+// under every frontier item and a top-down pass hands out depth-first
 // positions (an exclusive scan over the roots, then parent offset / parent
 // offset + left child count): the emitted pairs come out in exactly the order
-// of the recursive host traversal.
+// of the recursive host traversal, in whatever order a level holds its pairs.
 //
 // Buckets. Pair k = (a, b) gives the entries (dest a, src b) and (dest b,
 // src a); a stable LSD radix sort on the destination (8-bit digits, warp
@@ -75,102 +75,102 @@ __device__ int decide32(const Element &A, const Element &B, float e, float inv_m
     return A.area > B.area ? 1 : 2;
 }
 
-// decide every frontier pair in FP32 where that is certain: 0 link, 1 split
-// the first element, 2 the second; undecided pairs go to a list for FP64
-__global__ void __launch_bounds__(kThreads) k_decide32(int64_t n, const int2 *__restrict__ pairs, const uint16_t *__restrict__ root_level,
-                                                       int depth, const Element *__restrict__ el, float e, float inv_max_area,
-                                                       float inv_max_side, uint8_t *flag, int32_t *undecided,
-                                                       unsigned long long *n_undecided, int *max_level) {
-    int lvl = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i - (threadIdx.x) < n; i += (int64_t)gridDim.x * blockDim.x) {
-        int f = 0;
-        bool ok = i < n;
-        if (ok) {
-            int2 pr = pairs[i];
-            f = decide32(el[pr.x], el[pr.y], e, inv_max_area, inv_max_side);
-            flag[i] = (uint8_t)(f < 0 ? 0 : f);
-            lvl = max(lvl, (int)root_level[i] + depth);
-        }
-        // warp-aggregated append of the undecided pairs
-        unsigned m = __ballot_sync(0xffffffffu, ok && f < 0);
-        if (m) {
-            int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(n_undecided, (unsigned long long)__popc(m));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (ok && f < 0) undecided[base + __popc(m & ((1u << lane) - 1u))] = (int32_t)i;
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) lvl = max(lvl, __shfl_xor_sync(0xffffffffu, lvl, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(max_level, lvl);
-}
+// a level's counts on the device: pairs split, pairs for the FP64 test
+struct LevelCount {
+    unsigned long long splits, listed;
+};
 
-// the FP64 test (the host builder's own code) for the undecided pairs
-__global__ void __launch_bounds__(128) k_decide64(const unsigned long long *__restrict__ n_undecided, const int32_t *__restrict__ undecided,
-                                                  const int2 *__restrict__ pairs, const Element *__restrict__ el, double eps,
-                                                  double max_side, double max_area, uint8_t *flag) {
-    int64_t m = (int64_t)*n_undecided;
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m; j += (int64_t)gridDim.x * blockDim.x) {
-        int32_t i = undecided[j];
-        int2 pr = pairs[i];
-        flag[i] = (uint8_t)fcg_link_decision(el[pr.x], el[pr.y], eps, max_side, max_area);
+// The children of a warp's split pairs (f = 1 or 2: pair i splits its first
+// or second element; 0 a link; -1 none of this kernel's) into the next level,
+// at places that one atomic hands out; rank[i] says where (r: entries 2 r and
+// 2 r + 1; -1: a link).
+__device__ __forceinline__ void emit_children(LevelCount *count, int64_t ne, int64_t i, int f, int2 pr, uint16_t rl,
+                                              const Element *__restrict__ el, int32_t *__restrict__ rank, int64_t next_cap,
+                                              int2 *__restrict__ next, uint16_t *__restrict__ next_level, unsigned *bad) {
+    const unsigned split = __ballot_sync(0xffffffffu, f > 0);
+    if (f == 0) rank[i] = -1;
+    if (!split) return;
+    const int64_t r = warp_claim(&count->splits, __popc(split)) + __popc(split & ((1u << (threadIdx.x & 31)) - 1u));
+    if (f <= 0) return;
+    int2 c0 = pr, c1 = pr;
+    if (f == 1) {
+        c0.x = el[pr.x].left;
+        c1.x = el[pr.x].right;
+    } else {
+        c0.y = el[pr.y].left;
+        c1.y = el[pr.y].right;
     }
-}
-
-// per-tile count of split pairs
-__global__ void __launch_bounds__(kThreads) k_split_tiles(int64_t n, const uint8_t *__restrict__ flag, long long *tile_sums) {
-    __shared__ long long wt[32];
-    int64_t base = (int64_t)blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
-    long long splits = 0;
-    for (int j = 0; j < kItems; j++)
-        if (base + j < n) splits += flag[base + j] != 0;
-    splits = block_sum(splits, wt);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = splits;
-}
-
-// children of every split pair into the next level, at 2 * (exclusive rank)
-__global__ void __launch_bounds__(kThreads) k_expand(int64_t n, int64_t ne, const int2 *__restrict__ pairs,
-                                                     const uint16_t *__restrict__ root_level, const uint8_t *__restrict__ flag,
-                                                     const Element *__restrict__ el, const long long *__restrict__ tile_off,
-                                                     int32_t *rank, int2 *next, uint16_t *next_level, unsigned *bad) {
-    __shared__ long long wt[32];
-    int64_t base = (int64_t)blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
-    uint8_t f[kItems];
-    long long s = 0;
-    for (int j = 0; j < kItems; j++) {
-        f[j] = base + j < n ? flag[base + j] : 0;
-        s += f[j] != 0;
+    // a split side always has two children; anything else is a corrupt hierarchy
+    if (c0.x < 0 || c0.y < 0 || c1.x < 0 || c1.y < 0 || c0.x >= ne || c0.y >= ne || c1.x >= ne || c1.y >= ne) {
+        atomicAdd(bad, 1u);
+        c0 = c1 = make_int2(0, 0);
     }
-    long long tot;
-    long long r = block_exclusive_scan(s, wt, &tot) + tile_off[blockIdx.x];
-    for (int j = 0; j < kItems; j++) {
-        int64_t i = base + j;
-        if (i >= n) break;
-        if (!f[j]) {
-            rank[i] = -1;
-            continue;
-        }
-        int2 pr = pairs[i];
-        int2 c0 = pr, c1 = pr;
-        if (f[j] == 1) {
-            c0.x = el[pr.x].left;
-            c1.x = el[pr.x].right;
-        } else {
-            c0.y = el[pr.y].left;
-            c1.y = el[pr.y].right;
-        }
-        // a split side always has two children; anything else is a corrupt hierarchy
-        if (c0.x < 0 || c0.y < 0 || c1.x < 0 || c1.y < 0 || c0.x >= ne || c0.y >= ne || c1.x >= ne || c1.y >= ne) {
-            atomicAdd(bad, 1u);
-            c0 = c1 = make_int2(0, 0);
-        }
-        rank[i] = (int32_t)r;
+    rank[i] = (int32_t)r;
+    if (2 * r + 1 < next_cap) {  // always: the next level has room for two children of every pair
         next[2 * r] = c0;
         next[2 * r + 1] = c1;
-        uint16_t rl = root_level[i];
         next_level[2 * r] = rl;
         next_level[2 * r + 1] = rl;
-        r++;
+    }
+}
+
+// One level of the traversal: every pair is decided in FP32 where that is
+// certain (0 link, 1 split the first element, 2 the second) and its children
+// placed at once; the others are listed for k_link_level64. The pairs of this
+// level: n0, or twice the splits of the level before (read on the device, so
+// that several small levels run without the host).
+__global__ void __launch_bounds__(128) k_link_level(int64_t n0, const LevelCount *__restrict__ prev, const int2 *__restrict__ pairs,
+                                                    const uint16_t *__restrict__ root_level, int depth, int64_t ne,
+                                                    const Element *__restrict__ el, float e, float inv_max_area, float inv_max_side,
+                                                    int32_t *__restrict__ rank, int64_t next_cap, int2 *__restrict__ next,
+                                                    uint16_t *__restrict__ next_level, LevelCount *count, int32_t *__restrict__ listed,
+                                                    int *max_level, unsigned *bad) {
+    const int64_t n = prev ? 2 * (int64_t)prev->splits : n0;
+    const int lane = threadIdx.x & 31;
+    int lvl = 0;
+    // whole warps stay in the loop while their first pair exists (ballots below)
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i - lane < n; i += (int64_t)gridDim.x * blockDim.x) {
+        int f = -1;
+        bool undecided = false;
+        int2 pr = make_int2(0, 0);
+        uint16_t rl = 0;
+        if (i < n) {
+            pr = pairs[i];
+            rl = root_level[i];
+            lvl = max(lvl, (int)rl + depth);
+            f = decide32(el[pr.x], el[pr.y], e, inv_max_area, inv_max_side);
+            undecided = f < 0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, undecided);
+        if (m) {
+            const int64_t at = warp_claim(&count->listed, __popc(m)) + __popc(m & ((1u << lane) - 1u));
+            if (undecided) listed[at] = (int32_t)i;
+        }
+        emit_children(count, ne, i, f, pr, rl, el, rank, next_cap, next, next_level, bad);
+    }
+    for (int o = 16; o > 0; o >>= 1) lvl = max(lvl, __shfl_xor_sync(0xffffffffu, lvl, o));
+    if (lane == 0 && lvl) atomicMax(max_level, lvl);
+}
+
+// the FP64 test (the host builder's own code) for the level's listed pairs
+__global__ void __launch_bounds__(128) k_link_level64(const int2 *__restrict__ pairs, const uint16_t *__restrict__ root_level, int64_t ne,
+                                                      const Element *__restrict__ el, double eps, double max_side, double max_area,
+                                                      int32_t *__restrict__ rank, int64_t next_cap, int2 *__restrict__ next,
+                                                      uint16_t *__restrict__ next_level, LevelCount *count,
+                                                      const int32_t *__restrict__ listed, unsigned *bad) {
+    const int64_t m = (int64_t)count->listed;
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j - (threadIdx.x & 31) < m; j += (int64_t)gridDim.x * blockDim.x) {
+        int f = -1;
+        int64_t i = 0;
+        int2 pr = make_int2(0, 0);
+        uint16_t rl = 0;
+        if (j < m) {
+            i = listed[j];
+            pr = pairs[i];
+            rl = root_level[i];
+            f = fcg_link_decision(el[pr.x], el[pr.y], eps, max_side, max_area);
+        }
+        emit_children(count, ne, i, f, pr, rl, el, rank, next_cap, next, next_level, bad);
     }
 }
 
@@ -214,6 +214,9 @@ __global__ void k_entries(int64_t P, const int2 *__restrict__ pairs, const int32
 }
 
 // ------------------------------------------------------------------ host side
+constexpr size_t kMaxGroup = 24;       // levels launched at a time (the bound doubles: at most 18)
+constexpr int64_t kNoWait = 1 << 18;  // pairs up to which levels are launched without knowing their size
+
 struct Level {
     int64_t n = 0;
     int2 *pairs = nullptr;
@@ -254,12 +257,12 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const i
     long long *d_scalars;  // [0] scan total, [1] spare
     int *d_max_level;
     unsigned *d_bad;
-    unsigned long long *d_undecided;
-    const float inv_max_area = (float)(1.0 / max_area), inv_max_side = (float)(1.0 / max_side);
+    LevelCount *d_count;  // per level of a group
+    int32_t *d_listed = nullptr;
+    int64_t listed_room = 0;
     const bool trace = getenv("FCG_TRACE") != nullptr;
     const auto t_begin = std::chrono::steady_clock::now();
-    long long n_tests = 0, n_fp64 = 0;
-    LB_CK(B.alloc(&d_undecided, 1));
+    LB_CK(B.alloc(&d_count, kMaxGroup));
     LB_CK(B.alloc(&d_el, (size_t)ne));
     LB_CK(B.alloc(&d_node_of, (size_t)ne));
     LB_CK(B.alloc(&d_scalars, 2));
@@ -279,54 +282,71 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const i
         for (int64_t i = 0; i < n_roots; i++) h[(size_t)i] = make_int2(root_a[i], root_b[i]);
         LB_CK(B.alloc(&L0.pairs, (size_t)n_roots));
         LB_CK(B.alloc(&L0.root_level, (size_t)n_roots));
+        LB_CK(B.alloc(&L0.rank, (size_t)n_roots));
         LB_CK(cudaMemcpyAsync(L0.pairs, h.data(), (size_t)n_roots * sizeof(int2), cudaMemcpyHostToDevice, s));
         LB_CK(cudaMemcpyAsync(L0.root_level, root_level, (size_t)n_roots * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
     }
 
-    // frontier expansion, one level per step
-    for (int depth = 0;; depth++) {
-        Level &L = lv.back();
-        int64_t n = L.n;
-        unsigned tiles = grid_tiles(n);
-        uint8_t *flag;
-        long long *sums;
-        int32_t *undecided;
-        LB_CK(B.alloc(&flag, (size_t)n));
-        LB_CK(B.alloc(&sums, tiles));
-        LB_CK(B.alloc(&undecided, (size_t)n));
-        LB_CK(B.alloc(&L.rank, (size_t)n));
-        LB_CK(cudaMemsetAsync(d_undecided, 0, sizeof(unsigned long long), s));
-        k_decide32<<<grid_stride(n, sms), 256, 0, s>>>(n, L.pairs, L.root_level, depth, d_el, (float)eps, inv_max_area,
-                                                        inv_max_side, flag, undecided, d_undecided, d_max_level);
-        k_decide64<<<grid_stride(n, sms), 128, 0, s>>>(d_undecided, undecided, L.pairs, d_el, eps, max_side, max_area, flag);
-        k_split_tiles<<<tiles, kThreads, 0, s>>>(n, flag, sums);
-        k_scan_sums<<<1, 1024, 0, s>>>(tiles, sums, d_scalars);
-        LB_CK(cudaGetLastError());
-        long long level_counts[2] = {0, 0};  // splits, FP64 tests
-        LB_CK(cudaMemcpyAsync(&level_counts[0], d_scalars, sizeof(long long), cudaMemcpyDeviceToHost, s));
-        LB_CK(cudaMemcpyAsync(&level_counts[1], d_undecided, sizeof(long long), cudaMemcpyDeviceToHost, s));
-        LB_CK(cudaStreamSynchronize(s));
-        B.release(undecided);
-        long long splits = level_counts[0];
-        n_tests += n;
-        n_fp64 += level_counts[1];
-        if (splits > (1ll << 29)) {
-            err = "model too large for 32-bit link indices";
-            return FCG_OUT_OF_MEMORY;
-        }
-        Level nx;
-        nx.n = 2 * splits;
-        if (splits > 0) {
+    // frontier expansion, one level per launch. A level has at most twice the
+    // pairs of the one before: the host waits for the counts only when that
+    // bound has grown past kNoWait pairs since it last knew them.
+    long long n_tests = 0, n_fp64 = 0;
+    for (bool more = true; more;) {
+        const size_t first = lv.size() - 1;  // its size is known
+        int64_t bound = lv[first].n;
+        size_t d = first;
+        LB_CK(cudaMemsetAsync(d_count, 0, kMaxGroup * sizeof(LevelCount), s));
+        do {
+            if (bound > (1ll << 30)) {
+                err = "model too large for 32-bit link indices";
+                return FCG_OUT_OF_MEMORY;
+            }
+            if (bound > listed_room) {
+                B.release(d_listed);
+                listed_room = std::max<int64_t>(bound, kNoWait);
+                LB_CK(B.alloc(&d_listed, (size_t)listed_room));
+            }
+            Level nx;
+            nx.n = 2 * bound;
             LB_CK(B.alloc(&nx.pairs, (size_t)nx.n));
             LB_CK(B.alloc(&nx.root_level, (size_t)nx.n));
+            LB_CK(B.alloc(&nx.rank, (size_t)nx.n));
+            const Level &L = lv[d];
+            LevelCount *count = d_count + (d - first);
+            k_link_level<<<grid_stride(bound, sms, 128), 128, 0, s>>>(
+                L.n, d > first ? count - 1 : nullptr, L.pairs, L.root_level, (int)d, ne, d_el, (float)eps, (float)(1.0 / max_area),
+                (float)(1.0 / max_side), L.rank, nx.n, nx.pairs, nx.root_level, count, d_listed, d_max_level, d_bad);
+            k_link_level64<<<grid_stride(bound, sms, 128), 128, 0, s>>>(L.pairs, L.root_level, ne, d_el, eps, max_side, max_area, L.rank,
+                                                                       nx.n, nx.pairs, nx.root_level, count, d_listed, d_bad);
+            LB_CK(cudaGetLastError());
+            lv.push_back(nx);
+            d++;
+            bound *= 2;
+        } while (bound <= kNoWait && d - first < kMaxGroup);
+        std::vector<LevelCount> counts(d - first);
+        LB_CK(cudaMemcpyAsync(counts.data(), d_count, counts.size() * sizeof(LevelCount), cudaMemcpyDeviceToHost, s));
+        LB_CK(cudaStreamSynchronize(s));
+        for (size_t q = first; q < d; q++) {
+            const long long sp = (long long)counts[q - first].splits;
+            if (sp > (1ll << 29)) {
+                err = "model too large for 32-bit link indices";
+                return FCG_OUT_OF_MEMORY;
+            }
+            n_tests += lv[q].n;
+            n_fp64 += (long long)counts[q - first].listed;
+            B.release(lv[q].root_level);
+            lv[q + 1].n = 2 * sp;
+            if (sp == 0) {  // the traversal ended at level q
+                for (size_t u = q + 1; u <= d; u++) {
+                    B.release(lv[u].pairs);
+                    B.release(lv[u].root_level);
+                    B.release(lv[u].rank);
+                }
+                lv.resize(q + 1);
+                more = false;
+                break;
+            }
         }
-        k_expand<<<tiles, kThreads, 0, s>>>(n, ne, L.pairs, L.root_level, flag, d_el, sums, L.rank, nx.pairs, nx.root_level, d_bad);
-        LB_CK(cudaGetLastError());
-        B.release(flag);
-        B.release(sums);
-        B.release(L.root_level);
-        if (splits == 0) break;
-        lv.push_back(nx);
     }
     unsigned bad = 0;
     LB_CK(cudaMemcpyAsync(&bad, d_bad, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -350,9 +370,17 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const i
     if (trace) fprintf(stderr, "[fcg links]   traversal                    %9.3f ms\n",
                        std::chrono::duration<double, std::milli>(t_mark - t_begin).count());
     // links under every item, deepest level first
+    long long *cnt_all;
+    LB_CK(B.alloc(&cnt_all, (size_t)n_tests));
+    {
+        long long *at = cnt_all;
+        for (Level &L : lv) {
+            L.cnt = at;
+            at += L.n;
+        }
+    }
     for (size_t d = lv.size(); d-- > 0;) {
         Level &L = lv[d];
-        LB_CK(B.alloc(&L.cnt, (size_t)L.n));
         const long long *cn = d + 1 < lv.size() ? lv[d + 1].cnt : nullptr;
         k_count<<<grid_stride(L.n, sms), 256, 0, s>>>(L.n, L.rank, cn, L.cnt);
         LB_CK(cudaGetLastError());
@@ -387,8 +415,8 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const i
     for (Level &L : lv) {
         B.release(L.pairs);
         B.release(L.rank);
-        B.release(L.cnt);
     }
+    B.release(cnt_all);
 
     // rows: entries, degrees -> link_ptr, stable radix sort by destination
     const int64_t nent = 2 * P;

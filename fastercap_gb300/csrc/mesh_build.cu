@@ -11,13 +11,17 @@
 // internal element, including every element split along the way (`selfc`
 // on). The host builder reaches that closure depth first; here the pairs
 // advance one level per step:
-//   decide   every frontier pair in FP64 (the host builder's own code);
-//            non-split pairs update the largest achieved weight, split pairs
-//            mark a leaf to bisect
-//   number   the marked leaves by an exclusive scan (deterministic ids)
-//   bisect   the marked leaves; each new internal element adds the pair of
-//            its children, with `selfc`, to the next frontier
-//   expand   every split pair into its two children pairs.
+//   level    decide every frontier pair (FP32 where certain, else, from a
+//            list, by the host builder's own FP64 code); non-split pairs update
+//            the largest achieved weight; a split pair is listed for the next
+//            step, and the first one to split a leaf gives it the ids of its
+//            halves
+//   grow     the halves of every leaf given ids (its two halves are a pair of
+//            the next frontier, with `selfc`), and every listed pair's two
+//            children pairs.
+// Places in the next frontier and element ids come from one atomic per warp
+// and 32 pairs: no scans, and the host only waits where the next levels' sizes
+// have no useful bound.
 // The element ids differ from the host builder's (creation order), but the
 // tree, and so the flattened model, is the same. Recursion levels are those
 // of the host recursion: a conductor pair starts at level 1, the self pair of
@@ -50,6 +54,8 @@ constexpr int kMaxMeshLevel = 4096;           // the host recursion's limit
 constexpr uint16_t kSelfBit = kMeshSelfPair;  // frontier meta: self pass
 constexpr uint16_t kLevelMask = 0x7fff;       // frontier meta: recursion level
 constexpr int64_t kMaxFrontier = 1ll << 30;   // pairs held at once
+constexpr int64_t kNoWait = 1 << 18;          // pairs up to which levels are launched without knowing their size
+constexpr int kMaxGroup = 24;                 // levels launched at a time (the bound triples: at most 12)
 
 static_assert(sizeof(Element) == 96, "element record layout");
 
@@ -124,212 +130,188 @@ __device__ int mesh_decide32(const Element &A, const Element &B, bool selfc, flo
     return -1;
 }
 
-// Every frontier pair in FP32 where that is certain. Pairs the FP32 test
-// cannot decide go to a list for the FP64 test, and so do the kept pairs
-// that may hold the largest weight of the model: a kept pair whose upper
-// bound is below the largest lower bound already listed cannot (that listed
-// pair's exact weight is at least its lower bound), so only pairs near the
-// running maximum take the FP64 test for it. `lo_bits` holds that running
-// lower bound (bits of a non-negative double).
-__global__ void __launch_bounds__(128) k_mesh_decide32(int64_t n, const int2 *__restrict__ pairs, const uint16_t *__restrict__ meta,
-                                                       const Element *__restrict__ el, float e, float mesh_curv, float inv_max_area,
-                                                       float inv_max_side, uint8_t *flag, uint8_t *split, int32_t *listed,
-                                                       unsigned long long *n_listed, unsigned long long *lo_bits,
-                                                       int *max_level, unsigned *too_deep) {
+// what the levels know of one another, on the device
+struct LevelHead {
+    unsigned long long n, ne;                        // frontier pairs, elements
+    unsigned long long n_split, n_leaves, n_listed;  // pairs split, leaves bisected, pairs for the FP64 test
+};
+
+// a level's lists of split pairs (the side that splits in the sign of the
+// first id), of bisected leaves and of pairs for the FP64 test
+struct LevelLists {
+    int2 *split_pairs;
+    uint16_t *split_meta;
+    int32_t *leaves, *listed;
+};
+
+// A warp's split pairs (f = 1 or 2: the pair splits its first or second
+// element, a leaf when `leaf` is set) into the level's list; the first to
+// split a leaf gives it the ids of its halves.
+__device__ __forceinline__ void emit_splits(LevelHead *head, int64_t ne, int f, bool leaf, int2 pr, uint16_t m, Element *el, int *claim,
+                                            const LevelLists &ls) {
+    const unsigned split = __ballot_sync(0xffffffffu, f != 0);
+    if (!split) return;
+    const int x = f == 1 ? pr.x : pr.y;
+    const bool mine = f && leaf && atomicExch(&claim[x], 1) == 0;
+    const unsigned first = __ballot_sync(0xffffffffu, mine), below = (1u << (threadIdx.x & 31)) - 1u;
+    const int64_t rs = warp_claim(&head->n_split, __popc(split)) + __popc(split & below);
+    if (first) {
+        const int64_t rl = warp_claim(&head->n_leaves, __popc(first)) + __popc(first & below);
+        if (mine) {
+            ls.leaves[rl] = x;
+            el[x].left = (int32_t)(ne + 2 * rl);
+            el[x].right = (int32_t)(ne + 2 * rl + 1);
+        }
+    }
+    if (f) {
+        ls.split_pairs[rs] = make_int2(f == 2 ? ~pr.x : pr.x, pr.y);
+        ls.split_meta[rs] = m;
+    }
+}
+
+// One level's decisions in FP32 where that is certain. Pairs the FP32 test
+// cannot decide are listed for the FP64 test, and so are the kept pairs that
+// may hold the largest weight of the model: a kept pair whose upper bound is
+// below the largest lower bound already seen cannot (that pair's exact weight
+// is at least its lower bound), so only pairs near the running maximum take
+// the FP64 test for it. `lo_bits` holds that running lower bound (bits of a
+// non-negative double). With pre32 unset every pair takes the FP64 test.
+// A large level is bound by the gathers of its elements (96-byte records,
+// latency; four pairs a lane with one claim was slower, 218 -> 300 us a level
+// of 4M pairs), a small one by its launches: three kernels a level and a wait
+// for the host every few levels, instead of nine and one each: a 528-panel
+// model's refinement 1.74 -> 1.03 ms, its links 1.49 -> 0.90 ms.
+__global__ void __launch_bounds__(128, 6) k_mesh_level(LevelHead *__restrict__ head, const int2 *__restrict__ pairs,
+                                                       const uint16_t *__restrict__ meta, Element *el, int *claim, int pre32, float e,
+                                                       float mesh_curv, float inv_max_area, float inv_max_side, const LevelLists ls,
+                                                       unsigned long long *lo_bits, int *max_level, unsigned *too_deep) {
+    const int64_t n = (int64_t)head->n, ne = (int64_t)head->ne;
+    const int lane = threadIdx.x & 31;
     int lvl_max = 0;
     // whole warps stay in the loop while their first pair exists (ballots below)
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i - (threadIdx.x & 31) < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        bool ok = i < n, list = false;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i - lane < n; i += (int64_t)gridDim.x * blockDim.x) {
+        int f = 0;
+        bool leaf = false;
         double lo = 0.0;
-        if (ok) {
-            int2 pr = pairs[i];
-            uint16_t m = meta[i];
-            int lvl = m & kLevelMask;
+        int2 pr = make_int2(0, 0);
+        uint16_t m = 0;
+        if (i < n) {
+            pr = pairs[i];
+            m = meta[i];
+            const int lvl = m & kLevelMask;
             lvl_max = max(lvl_max, lvl);
             if (lvl > kMaxMeshLevel) {
                 atomicOr(too_deep, 1u);
-                flag[i] = 0;
-            } else {
+            } else if (pre32) {
                 const Element &A = el[pr.x], &B = el[pr.y];
                 float c1 = 0, e1 = 0, c2 = 0, e2 = 0;
-                int f = mesh_decide32(A, B, (m & kSelfBit) != 0, e, mesh_curv, inv_max_area, inv_max_side, c1, e1, c2, e2);
-                flag[i] = (uint8_t)(f < 0 ? 0 : f);
-                if (f > 0) {
-                    int x = f == 1 ? pr.x : pr.y;
-                    if (el[x].type & FCG_IS_LEAF) split[x] = 1;
-                } else if (f < 0) {
-                    list = true;
-                } else {
+                f = mesh_decide32(A, B, (m & kSelfBit) != 0, e, mesh_curv, inv_max_area, inv_max_side, c1, e1, c2, e2);
+                leaf = ((f == 1 ? A.type : B.type) & FCG_IS_LEAF) != 0;
+                if (f == 0) {
                     // a kept pair: may its exact weight be the model's largest?
                     float hi = 0.0f, l = 0.0f;
                     if (!(A.type & FCG_IS_SUPER_NODE)) { hi = c1 + e1; l = c1 - e1; }
                     if (!(B.type & FCG_IS_SUPER_NODE)) { hi = fmaxf(hi, c2 + e2); l = fmaxf(l, c2 - e2); }
-                    double cur = __longlong_as_double((long long)*(volatile unsigned long long *)lo_bits);
+                    const double cur = __longlong_as_double((long long)*(volatile unsigned long long *)lo_bits);
                     if (hi > 0.0f && (double)hi >= cur) {
-                        list = true;
-                        lo = l > 0.0f ? (double)l : 0.0;
+                        f = -1;
+                        if (l > 0.0f) lo = (double)l;
                     }
                 }
+            } else {
+                f = -1;
             }
         }
-        // warp-aggregated append to the FP64 list, and the running lower bound
-        unsigned mk = __ballot_sync(0xffffffffu, list);
-        if (mk) {
-            int lane = threadIdx.x & 31, leader = __ffs(mk) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(n_listed, (unsigned long long)__popc(mk));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (list) listed[base + __popc(mk & ((1u << lane) - 1u))] = (int32_t)i;
+        const unsigned listed = __ballot_sync(0xffffffffu, f < 0);
+        if (listed) {
+            const int64_t at = warp_claim(&head->n_listed, __popc(listed)) + __popc(listed & ((1u << lane) - 1u));
+            if (f < 0) ls.listed[at] = (int32_t)i;
             for (int o = 16; o > 0; o >>= 1) lo = fmax(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-            if (lane == leader && lo > 0.0) atomicMax(lo_bits, (unsigned long long)__double_as_longlong(lo));
+            if (lane == 0 && lo > 0.0) atomicMax(lo_bits, (unsigned long long)__double_as_longlong(lo));
         }
+        emit_splits(head, ne, max(f, 0), leaf, pr, m, el, claim, ls);
     }
     for (int o = 16; o > 0; o >>= 1) lvl_max = max(lvl_max, __shfl_xor_sync(0xffffffffu, lvl_max, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(max_level, lvl_max);
+    if (lane == 0 && lvl_max) atomicMax(max_level, lvl_max);
 }
 
-// the FP64 test (the host builder's own code) for the listed pairs: the
-// decision and, for kept pairs, the exact weights behind the model's largest
-__global__ void __launch_bounds__(128) k_mesh_decide64(const unsigned long long *__restrict__ n_listed,
-                                                       const int32_t *__restrict__ listed, const int2 *__restrict__ pairs,
-                                                       const uint16_t *__restrict__ meta, const Element *__restrict__ el,
-                                                       double mesh_eps, double mesh_curv, double max_side, double max_area,
-                                                       uint8_t *flag, uint8_t *split, unsigned long long *max_eps_bits) {
-    int64_t cnt = (int64_t)*n_listed;
+// The FP64 test (the host builder's own code) of the level's listed pairs: the
+// decision and, for kept pairs, the exact weights behind the model's largest.
+__global__ void __launch_bounds__(128) k_mesh_level64(LevelHead *__restrict__ head, const int2 *__restrict__ pairs,
+                                                      const uint16_t *__restrict__ meta, Element *el, int *claim, double mesh_eps,
+                                                      double mesh_curv, double max_side, double max_area, const LevelLists ls,
+                                                      unsigned long long *max_eps_bits) {
+    const int64_t cnt = (int64_t)head->n_listed, ne = (int64_t)head->ne;
+    // largest weight of the pairs this thread kept, as the bits of a
+    // non-negative double (their order is the values' order)
     unsigned long long eps_max = 0;
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += (int64_t)gridDim.x * blockDim.x) {
-        int64_t i = listed[j];
-        int2 pr = pairs[i];
-        const Element &A = el[pr.x], &B = el[pr.y];
-        double c1, c2;
-        int f = fcg_mesh_decision(A, B, (meta[i] & kSelfBit) != 0, mesh_eps, mesh_curv, max_side, max_area, &c1, &c2);
-        flag[i] = (uint8_t)f;
-        if (f) {
-            int x = f == 1 ? pr.x : pr.y;
-            if (el[x].type & FCG_IS_LEAF) split[x] = 1;
-        } else {
-            if (!(A.type & FCG_IS_SUPER_NODE) && c1 == c1) eps_max = max(eps_max, (unsigned long long)__double_as_longlong(c1));
-            if (!(B.type & FCG_IS_SUPER_NODE) && c2 == c2) eps_max = max(eps_max, (unsigned long long)__double_as_longlong(c2));
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j - (threadIdx.x & 31) < cnt; j += (int64_t)gridDim.x * blockDim.x) {
+        int f = 0;
+        bool leaf = false;
+        int2 pr = make_int2(0, 0);
+        uint16_t m = 0;
+        if (j < cnt) {
+            const int64_t i = ls.listed[j];
+            pr = pairs[i];
+            m = meta[i];
+            const Element &A = el[pr.x], &B = el[pr.y];
+            double c1, c2;
+            f = fcg_mesh_decision(A, B, (m & kSelfBit) != 0, mesh_eps, mesh_curv, max_side, max_area, &c1, &c2);
+            leaf = ((f == 1 ? A.type : B.type) & FCG_IS_LEAF) != 0;
+            if (!f) {
+                if (!(A.type & FCG_IS_SUPER_NODE) && c1 == c1) eps_max = max(eps_max, (unsigned long long)__double_as_longlong(c1));
+                if (!(B.type & FCG_IS_SUPER_NODE) && c2 == c2) eps_max = max(eps_max, (unsigned long long)__double_as_longlong(c2));
+            }
         }
+        emit_splits(head, ne, f, leaf, pr, m, el, claim, ls);
     }
     for (int o = 16; o > 0; o >>= 1) eps_max = max(eps_max, __shfl_xor_sync(0xffffffffu, eps_max, o));
     if ((threadIdx.x & 31) == 0 && eps_max) atomicMax(max_eps_bits, eps_max);
 }
 
-__global__ void __launch_bounds__(128) k_mesh_decide(int64_t n, const int2 *__restrict__ pairs, const uint16_t *__restrict__ meta,
-                                                     const Element *__restrict__ el, double mesh_eps, double mesh_curv,
-                                                     double max_side, double max_area, uint8_t *flag, uint8_t *split,
-                                                     unsigned long long *max_eps_bits, int *max_level, unsigned *too_deep) {
-    int lvl_max = 0;
-    // largest weight of the pairs this thread kept, as the bits of a
-    // non-negative double (their order is the values' order); one atomic per
-    // warp at the end instead of one per pair on a single word
-    unsigned long long eps_max = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        int2 pr = pairs[i];
-        uint16_t m = meta[i];
-        int lvl = m & kLevelMask;
-        lvl_max = max(lvl_max, lvl);
-        if (lvl > kMaxMeshLevel) {
-            atomicOr(too_deep, 1u);
-            flag[i] = 0;
-            continue;
-        }
-        const Element &A = el[pr.x], &B = el[pr.y];
-        double c1, c2;
-        int f = fcg_mesh_decision(A, B, (m & kSelfBit) != 0, mesh_eps, mesh_curv, max_side, max_area, &c1, &c2);
-        flag[i] = (uint8_t)f;
-        if (f) {
-            int x = f == 1 ? pr.x : pr.y;
-            if (el[x].type & FCG_IS_LEAF) split[x] = 1;  // many pairs may mark the same leaf
+// The next frontier: the children of every split pair (2 r, 2 r + 1), then the
+// halves of every bisected leaf, which are made here; and the next level's head.
+__global__ void __launch_bounds__(256) k_mesh_grow(LevelHead *__restrict__ head, Element *el, int32_t *depth,
+                                                   const LevelLists ls, int2 *__restrict__ next, uint16_t *__restrict__ next_meta) {
+    const int64_t ns = (int64_t)head->n_split, nlv = (int64_t)head->n_leaves, ne = (int64_t)head->ne;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        head[1].n = (unsigned long long)(2 * ns + nlv);
+        head[1].ne = (unsigned long long)(ne + 2 * nlv);
+    }
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ns + nlv; t += (int64_t)gridDim.x * blockDim.x) {
+        if (t < ns) {
+            int2 p = ls.split_pairs[t];
+            const bool second = p.x < 0;
+            if (second) p.x = ~p.x;
+            int2 c0 = p, c1 = p;
+            if (second) {
+                c0.y = el[p.y].left;
+                c1.y = el[p.y].right;
+            } else {
+                c0.x = el[p.x].left;
+                c1.x = el[p.x].right;
+            }
+            const uint16_t m = ls.split_meta[t];
+            const uint16_t m1 = (uint16_t)((m & kSelfBit) | (uint16_t)min((m & kLevelMask) + 1, (int)kLevelMask));
+            next[2 * t] = c0;
+            next[2 * t + 1] = c1;
+            next_meta[2 * t] = m1;
+            next_meta[2 * t + 1] = m1;
         } else {
-            // the largest weight of a pair that needed no refinement (weights are >= 0)
-            if (!(A.type & FCG_IS_SUPER_NODE) && c1 == c1) eps_max = max(eps_max, (unsigned long long)__double_as_longlong(c1));
-            if (!(B.type & FCG_IS_SUPER_NODE) && c2 == c2) eps_max = max(eps_max, (unsigned long long)__double_as_longlong(c2));
+            const int64_t k = t - ns;
+            const int32_t x = ls.leaves[k], l = (int32_t)(ne + 2 * k), r = l + 1;
+            Element Lc, Rc;
+            fcg_subdivide(el[x], Lc, Rc);
+            el[l] = Lc;
+            el[r] = Rc;
+            const int32_t d = depth[x];
+            depth[l] = d + 1;
+            depth[r] = d + 1;
+            el[x].type = (uint8_t)(el[x].type & ~FCG_IS_LEAF);
+            next[2 * ns + k] = make_int2(l, r);
+            next_meta[2 * ns + k] = (uint16_t)(kSelfBit | (uint16_t)min(d + 2, (int)kLevelMask));
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        lvl_max = max(lvl_max, __shfl_xor_sync(0xffffffffu, lvl_max, o));
-        eps_max = max(eps_max, __shfl_xor_sync(0xffffffffu, eps_max, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(max_level, lvl_max);
-        if (eps_max) atomicMax(max_eps_bits, eps_max);
-    }
-}
-
-// bisect the marked leaves into ids ne + 2 rank, ne + 2 rank + 1; the pair of
-// the two halves joins the next frontier (self pass) after the split pairs'
-// children
-__global__ void k_mesh_bisect(int64_t ne, uint8_t *split, const int32_t *__restrict__ rank, Element *el, int32_t *depth,
-                              int64_t child_base, int2 *next, uint16_t *next_meta) {
-    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < ne; x += (int64_t)gridDim.x * blockDim.x) {
-        if (!split[x]) continue;
-        split[x] = 0;
-        int64_t k = rank[x];
-        int32_t l = (int32_t)(ne + 2 * k), r = l + 1;
-        Element P = el[x];
-        Element Lc, Rc;
-        fcg_subdivide(P, Lc, Rc);
-        el[l] = Lc;
-        el[r] = Rc;
-        int32_t d = depth[x];
-        depth[l] = d + 1;
-        depth[r] = d + 1;
-        el[x].left = l;
-        el[x].right = r;
-        el[x].type = (uint8_t)(P.type & ~FCG_IS_LEAF);
-        next[child_base + k] = make_int2(l, r);
-        next_meta[child_base + k] = (uint16_t)(kSelfBit | (uint16_t)min(d + 2, (int)kLevelMask));
-    }
-}
-
-// children of every split pair at 2 * (exclusive rank among split pairs)
-__global__ void __launch_bounds__(kThreads) k_mesh_expand(int64_t n, const int2 *__restrict__ pairs, const uint16_t *__restrict__ meta,
-                                                          const uint8_t *__restrict__ flag, const Element *__restrict__ el,
-                                                          const long long *__restrict__ tile_off, int2 *next, uint16_t *next_meta) {
-    __shared__ long long wt[32];
-    int64_t base = (int64_t)blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
-    uint8_t f[kItems];
-    long long s = 0;
-    for (int j = 0; j < kItems; j++) {
-        f[j] = base + j < n ? flag[base + j] : 0;
-        s += f[j] != 0;
-    }
-    long long tot;
-    long long r = block_exclusive_scan(s, wt, &tot) + tile_off[blockIdx.x];
-    for (int j = 0; j < kItems; j++) {
-        int64_t i = base + j;
-        if (i >= n) break;
-        if (!f[j]) continue;
-        int2 pr = pairs[i];
-        int2 c0 = pr, c1 = pr;
-        if (f[j] == 1) {
-            c0.x = el[pr.x].left;
-            c1.x = el[pr.x].right;
-        } else {
-            c0.y = el[pr.y].left;
-            c1.y = el[pr.y].right;
-        }
-        uint16_t m = meta[i];
-        uint16_t m1 = (uint16_t)((m & kSelfBit) | (uint16_t)min((m & kLevelMask) + 1, (int)kLevelMask));
-        next[2 * r] = c0;
-        next[2 * r + 1] = c1;
-        next_meta[2 * r] = m1;
-        next_meta[2 * r + 1] = m1;
-        r++;
-    }
-}
-
-__global__ void k_count_split(int64_t n, const uint8_t *__restrict__ flag, long long *tile_sums) {
-    __shared__ long long wt[32];
-    int64_t base = (int64_t)blockIdx.x * kTile + (int64_t)threadIdx.x * kItems;
-    long long c = 0;
-    for (int j = 0; j < kItems; j++)
-        if (base + j < n) c += flag[base + j] != 0;
-    c = block_sum(c, wt);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = c;
 }
 
 }  // namespace
@@ -359,131 +341,151 @@ int mesh_refine_device(DeviceContext &ctx, std::vector<Element> &el, const std::
     int64_t ne = (int64_t)el.size();
     int64_t cap = std::max<int64_t>(2 * ne, ne + (1 << 20));
     Element *d_el;
-    int32_t *d_depth, *d_rank;
-    uint8_t *d_split;
-    long long *d_scalars;  // [0] split pairs, [1] marked leaves
-    unsigned long long *d_max_eps, *d_lo_bits, *d_n_listed;
+    int32_t *d_depth;
+    int *d_claim;
+    LevelHead *d_head;
+    unsigned long long *d_max_eps, *d_lo_bits;
     int *d_max_level;
     unsigned *d_too_deep;
     MB_CK(B.alloc(&d_el, (size_t)cap));
     MB_CK(B.alloc(&d_depth, (size_t)cap));
-    MB_CK(B.alloc(&d_rank, (size_t)cap));
-    MB_CK(B.alloc(&d_split, (size_t)cap));
-    MB_CK(B.alloc(&d_scalars, 2));
+    MB_CK(B.alloc(&d_claim, (size_t)cap));
+    MB_CK(B.alloc(&d_head, (size_t)kMaxGroup + 1));
     MB_CK(B.alloc(&d_max_eps, 1));
     MB_CK(B.alloc(&d_lo_bits, 1));
-    MB_CK(B.alloc(&d_n_listed, 1));
     MB_CK(B.alloc(&d_max_level, 1));
     MB_CK(B.alloc(&d_too_deep, 1));
     MB_CK(cudaMemcpyAsync(d_el, el.data(), (size_t)ne * sizeof(Element), cudaMemcpyHostToDevice, s));
     MB_CK(cudaMemcpyAsync(d_depth, depth.data(), (size_t)ne * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    MB_CK(cudaMemsetAsync(d_split, 0, (size_t)cap, s));
+    MB_CK(cudaMemsetAsync(d_claim, 0, (size_t)cap * sizeof(int), s));
     MB_CK(cudaMemsetAsync(d_max_eps, 0, sizeof(unsigned long long), s));
     MB_CK(cudaMemsetAsync(d_lo_bits, 0, sizeof(unsigned long long), s));
     MB_CK(cudaMemsetAsync(d_max_level, 0, sizeof(int), s));
     MB_CK(cudaMemsetAsync(d_too_deep, 0, sizeof(unsigned), s));
 
     int64_t n = (int64_t)root_a.size();
-    int2 *pairs = nullptr;
-    uint16_t *meta = nullptr;
+    // two frontiers, and the split pairs and bisected leaves of a level
+    int2 *pairs[2] = {nullptr, nullptr};
+    uint16_t *meta[2] = {nullptr, nullptr};
+    LevelLists ls = {nullptr, nullptr, nullptr, nullptr};
+    int64_t room[2] = {0, 0}, list_room = 0;
+    auto frontier = [&](int f, int64_t need) -> cudaError_t {
+        if (need <= room[f]) return cudaSuccess;
+        B.release(pairs[f]);
+        B.release(meta[f]);
+        room[f] = std::max<int64_t>(need, 1 << 16);
+        cudaError_t e = B.alloc(&pairs[f], (size_t)room[f]);
+        return e == cudaSuccess ? B.alloc(&meta[f], (size_t)room[f]) : e;
+    };
+    auto lists = [&](int64_t need) -> cudaError_t {
+        if (need <= list_room) return cudaSuccess;
+        B.release(ls.split_pairs);
+        B.release(ls.split_meta);
+        B.release(ls.leaves);
+        B.release(ls.listed);
+        list_room = std::max<int64_t>(need, 1 << 16);
+        cudaError_t e = B.alloc(&ls.split_pairs, (size_t)list_room);
+        if (e == cudaSuccess) e = B.alloc(&ls.split_meta, (size_t)list_room);
+        if (e == cudaSuccess) e = B.alloc(&ls.leaves, (size_t)list_room);
+        return e == cudaSuccess ? B.alloc(&ls.listed, (size_t)list_room) : e;
+    };
+    // room for elements: the arrays grow, keeping the first `have`
+    auto elements = [&](int64_t have, int64_t need) -> cudaError_t {
+        if (need <= cap) return cudaSuccess;
+        const int64_t ncap = std::max<int64_t>(2 * cap, need);
+        Element *el2;
+        int32_t *depth2;
+        int *claim2;
+        cudaError_t e = B.alloc(&el2, (size_t)ncap);
+        if (e == cudaSuccess) e = B.alloc(&depth2, (size_t)ncap);
+        if (e == cudaSuccess) e = B.alloc(&claim2, (size_t)ncap);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(el2, d_el, (size_t)have * sizeof(Element), cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(depth2, d_depth, (size_t)have * sizeof(int32_t), cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(claim2, d_claim, (size_t)have * sizeof(int), cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(claim2 + have, 0, (size_t)(ncap - have) * sizeof(int), s);
+        if (e != cudaSuccess) return e;
+        B.release(d_el);
+        B.release(d_depth);
+        B.release(d_claim);
+        d_el = el2;
+        d_depth = depth2;
+        d_claim = claim2;
+        cap = ncap;
+        return cudaSuccess;
+    };
     {
         std::vector<int2> h((size_t)n);
         for (int64_t i = 0; i < n; i++) h[(size_t)i] = make_int2(root_a[(size_t)i], root_b[(size_t)i]);
-        MB_CK(B.alloc(&pairs, (size_t)n));
-        MB_CK(B.alloc(&meta, (size_t)n));
-        MB_CK(cudaMemcpyAsync(pairs, h.data(), (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, s));
-        MB_CK(cudaMemcpyAsync(meta, root_meta.data(), (size_t)n * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
+        MB_CK(frontier(0, n));
+        MB_CK(cudaMemcpyAsync(pairs[0], h.data(), (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, s));
+        MB_CK(cudaMemcpyAsync(meta[0], root_meta.data(), (size_t)n * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
         MB_CK(cudaStreamSynchronize(s));  // the host vector goes out of scope
     }
     long long tests = 0, steps = 0;
+    int cur = 0;
+    auto grid_of = [&](int64_t items, int per) {
+        return (unsigned)std::max<int64_t>(std::min<int64_t>((items + per - 1) / per, (int64_t)sms * 16), 1);
+    };
     while (n > 0) {
-        steps++;
-        tests += n;
-        uint8_t *flag;
-        int32_t *listed;
-        long long *tsums, *esums;
-        unsigned tiles = grid_tiles(n), etiles = grid_tiles(ne);
-        MB_CK(B.alloc(&flag, (size_t)n));
-        MB_CK(B.alloc(&listed, (size_t)n));
-        MB_CK(B.alloc(&tsums, tiles));
-        MB_CK(B.alloc(&esums, etiles));
-        if (fp64_only) {
-            k_mesh_decide<<<grid_stride(n, sms, 128), 128, 0, s>>>(n, pairs, meta, d_el, mesh_eps, mesh_curv, max_side, max_area,
-                                                                   flag, d_split, d_max_eps, d_max_level, d_too_deep);
-        } else {
-            // FP32 pre-test, then the FP64 test for the listed pairs
-            MB_CK(cudaMemsetAsync(d_n_listed, 0, sizeof(unsigned long long), s));
-            k_mesh_decide32<<<grid_stride(n, sms, 128), 128, 0, s>>>(n, pairs, meta, d_el, (float)mesh_eps, (float)mesh_curv,
-                                                                     (float)(1.0 / max_area), (float)(1.0 / max_side), flag,
-                                                                     d_split, listed, d_n_listed, d_lo_bits, d_max_level,
-                                                                     d_too_deep);
-            k_mesh_decide64<<<grid_stride(n, sms, 128), 128, 0, s>>>(d_n_listed, listed, pairs, meta, d_el, mesh_eps, mesh_curv,
-                                                                     max_side, max_area, flag, d_split, d_max_eps);
-        }
-        k_count_split<<<tiles, kThreads, 0, s>>>(n, flag, tsums);
-        k_scan_sums<<<1, 1024, 0, s>>>(tiles, tsums, d_scalars);
-        exclusive_scan(s, ne, d_split, d_rank, esums, d_scalars + 1);
-        MB_CK(cudaGetLastError());
-        long long h[2];
+        // levels are launched without waiting while the bound on their size
+        // (every pair split, each by a leaf's bisection: three next pairs, two
+        // elements) stays below kNoWait; above it the host waits for a level's
+        // counts before it makes room for the next
+        std::vector<LevelHead> heads(kMaxGroup + 1, LevelHead{0, 0, 0, 0, 0});
+        heads[0].n = (unsigned long long)n;
+        heads[0].ne = (unsigned long long)ne;
+        MB_CK(cudaMemcpyAsync(d_head, heads.data(), heads.size() * sizeof(LevelHead), cudaMemcpyHostToDevice, s));
+        int64_t bound = n, ne_bound = ne;
+        int g = 0;
+        bool waited = false;
+        do {
+            LevelHead *head = d_head + g;
+            MB_CK(lists(bound));
+            k_mesh_level<<<grid_of(bound, 128), 128, 0, s>>>(head, pairs[cur], meta[cur], d_el, d_claim,
+                                                                       fp64_only ? 0 : 1, (float)mesh_eps, (float)mesh_curv,
+                                                                       (float)(1.0 / max_area), (float)(1.0 / max_side), ls,
+                                                                       d_lo_bits, d_max_level, d_too_deep);
+            k_mesh_level64<<<grid_of(bound, 128), 128, 0, s>>>(head, pairs[cur], meta[cur], d_el, d_claim, mesh_eps, mesh_curv,
+                                                              max_side, max_area, ls, d_max_eps);
+            int64_t next_bound = 3 * bound, grow = 2 * bound;
+            if (next_bound > kNoWait) {
+                LevelHead h;
+                unsigned deep = 0;
+                MB_CK(cudaMemcpyAsync(&h, head, sizeof h, cudaMemcpyDeviceToHost, s));
+                MB_CK(cudaMemcpyAsync(&deep, d_too_deep, sizeof deep, cudaMemcpyDeviceToHost, s));
+                MB_CK(cudaStreamSynchronize(s));
+                waited = true;
+                next_bound = (int64_t)(2 * h.n_split + h.n_leaves);
+                grow = (int64_t)(2 * h.n_leaves);
+                ne_bound = (int64_t)h.ne;
+                if (deep || next_bound > kMaxFrontier || ne_bound + grow > 0x7fffffffLL) {
+                    err = "mesh refinement recursion too deep (touching or overlapping panels?)";
+                    return FCG_GENERIC_ERROR;
+                }
+            }
+            MB_CK(frontier(cur ^ 1, next_bound));
+            MB_CK(elements(ne_bound, ne_bound + grow));
+            k_mesh_grow<<<grid_of(waited ? std::max<int64_t>(next_bound, 1) : 2 * bound, 256), 256, 0, s>>>(
+                head, d_el, d_depth, ls, pairs[cur ^ 1], meta[cur ^ 1]);
+            MB_CK(cudaGetLastError());
+            cur ^= 1;
+            bound = next_bound;
+            ne_bound += grow;
+            steps++;
+            g++;
+        } while (!waited && bound <= kNoWait && g < kMaxGroup);
+        heads.resize((size_t)g + 1);
         unsigned deep = 0;
-        MB_CK(cudaMemcpyAsync(h, d_scalars, 2 * sizeof(long long), cudaMemcpyDeviceToHost, s));
+        MB_CK(cudaMemcpyAsync(heads.data(), d_head, heads.size() * sizeof(LevelHead), cudaMemcpyDeviceToHost, s));
         MB_CK(cudaMemcpyAsync(&deep, d_too_deep, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         MB_CK(cudaStreamSynchronize(s));
         if (deep) {
             err = "mesh refinement recursion too deep (touching or overlapping panels?)";
             return FCG_GENERIC_ERROR;
         }
-        const long long n_split_pairs = h[0], n_leaves = h[1];
-        const int64_t n_next = 2 * n_split_pairs + n_leaves;
-        if (n_next > kMaxFrontier || ne + 2 * n_leaves > 0x7fffffffLL) {
-            err = "mesh refinement recursion too deep (touching or overlapping panels?)";
-            return FCG_GENERIC_ERROR;
-        }
-        if (ne + 2 * n_leaves > cap) {  // grow the element arrays
-            int64_t ncap = std::max<int64_t>(2 * cap, ne + 2 * n_leaves);
-            Element *el2;
-            int32_t *depth2, *rank2;
-            uint8_t *split2;
-            MB_CK(B.alloc(&el2, (size_t)ncap));
-            MB_CK(B.alloc(&depth2, (size_t)ncap));
-            MB_CK(B.alloc(&rank2, (size_t)ncap));
-            MB_CK(B.alloc(&split2, (size_t)ncap));
-            MB_CK(cudaMemcpyAsync(el2, d_el, (size_t)ne * sizeof(Element), cudaMemcpyDeviceToDevice, s));
-            MB_CK(cudaMemcpyAsync(depth2, d_depth, (size_t)ne * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-            MB_CK(cudaMemcpyAsync(rank2, d_rank, (size_t)ne * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-            MB_CK(cudaMemcpyAsync(split2, d_split, (size_t)ne, cudaMemcpyDeviceToDevice, s));
-            MB_CK(cudaMemsetAsync(split2 + ne, 0, (size_t)(ncap - ne), s));
-            B.release(d_el);
-            B.release(d_depth);
-            B.release(d_rank);
-            B.release(d_split);
-            d_el = el2;
-            d_depth = depth2;
-            d_rank = rank2;
-            d_split = split2;
-            cap = ncap;
-        }
-        int2 *next = nullptr;
-        uint16_t *next_meta = nullptr;
-        if (n_next > 0) {
-            MB_CK(B.alloc(&next, (size_t)n_next));
-            MB_CK(B.alloc(&next_meta, (size_t)n_next));
-        }
-        if (n_leaves > 0)
-            k_mesh_bisect<<<grid_stride(ne, sms), 256, 0, s>>>(ne, d_split, d_rank, d_el, d_depth, 2 * n_split_pairs, next,
-                                                               next_meta);
-        if (n_split_pairs > 0) k_mesh_expand<<<tiles, kThreads, 0, s>>>(n, pairs, meta, flag, d_el, tsums, next, next_meta);
-        MB_CK(cudaGetLastError());
-        B.release(flag);
-        B.release(listed);
-        B.release(tsums);
-        B.release(esums);
-        B.release(pairs);
-        B.release(meta);
-        pairs = next;
-        meta = next_meta;
-        ne += 2 * n_leaves;
-        n = n_next;
+        for (size_t q = 0; q + 1 < heads.size(); q++) tests += (long long)heads[q].n;
+        n = (int64_t)heads.back().n;
+        ne = (int64_t)heads.back().ne;
     }
     unsigned long long eps_bits = 0;
     MB_CK(cudaMemcpyAsync(&eps_bits, d_max_eps, sizeof(eps_bits), cudaMemcpyDeviceToHost, s));

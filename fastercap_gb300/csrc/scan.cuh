@@ -49,6 +49,14 @@ __device__ T block_exclusive_scan(T v, T *warp_tot, T *total) {
     return before + x - v;
 }
 
+// the warp's `total` places of a global list: one atomic, the first place to
+// every lane
+__device__ __forceinline__ int64_t warp_claim(unsigned long long *count, int total) {
+    unsigned long long base = 0;
+    if ((threadIdx.x & 31) == 0 && total) base = atomicAdd(count, (unsigned long long)total);
+    return (int64_t)__shfl_sync(0xffffffffu, base, 0);
+}
+
 template <class T>
 __device__ T block_sum(T v, T *warp_tot) {
     T total;
