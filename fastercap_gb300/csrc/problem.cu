@@ -237,6 +237,7 @@ struct DeviceProblem {
     // near-field (band 0) link list, built on the first fill
     int64_t n_near = -1;
     int32_t *near_link = NULL, *near_row = NULL;
+    int32_t *near_fp64 = NULL;  // mixed fill: near-list entries the FP64 formula decides (made by the first fill)
     fcg_tri64 *tri = NULL;    // source-triangle tables for the FP64 near field
     fcg_quad64 *quad = NULL;  // and for the FP64 far field
     fcg_tri32 *tri32 = NULL;  // scaled FP32 tables for the mixed near field and self terms
@@ -861,12 +862,20 @@ __device__ __noinline__ double self_fp64(const float *c, const float *v) {
 
 // Mixed-precision near-field links: the analytic potential in FP32 in the
 // source triangle's scaled frame (fcg_pot_near32), one thread per listed
-// link; a link whose guard FP32 cannot decide takes the FP64 formula. Held
-// to 64 registers (eight 128-thread CTAs per SM): the few spills cost less
-// than the occupancy they buy (sphere fill 0.86 -> 0.77 ms).
+// link. A link whose guard FP32 cannot decide takes the FP64 formula: with
+// LIST set it is listed for k_fill_near_fp64, because one such lane holds its
+// whole warp on a pipe that takes 20 cycles an instruction (under 1 % of the
+// links were most of the time: 28.5M links, 20 thousand listed 866 -> 271 us
+// for both kernels, the batch of six 1822 -> 524, 1.1M links 135 -> 72). Models with
+// dielectric panels decide in place: there the list gains nothing (20M links
+// 249 and 238 us), and the central differences of a dielectric coefficient
+// show how a kernel's compilation contracts its last bit (2e-4 of a few
+// coefficients, 2e-8 of the matrix). Held to 64 registers (eight 128-thread CTAs per SM): the
+// few spills cost less than the occupancy they buy (sphere fill 0.86 -> 0.77 ms).
+template <bool LIST>
 __global__ void __launch_bounds__(128, 8) k_fill_near32(int64_t n, const int32_t *__restrict__ near_link, const int32_t *__restrict__ near_row,
                               const uint32_t *__restrict__ src, const NodeGeo *__restrict__ geo, const fcg_tri32 *__restrict__ tri,
-                              float *__restrict__ c32, unsigned *status, unsigned long long *fb) {
+                              float *__restrict__ c32, unsigned *status, unsigned long long *fb, int32_t *__restrict__ listed) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
         int64_t l = near_link[t];
         const NodeGeo &g1 = geo[near_row[t]];
@@ -874,9 +883,28 @@ __global__ void __launch_bounds__(128, 8) k_fill_near32(int64_t n, const int32_t
         const NodeGeo &g2 = geo[j];
         float val;
         if (!fcg_pot_near32(g1.type, g1.c, g1.n, g2.c, tri[j], &val)) {
+            if constexpr (LIST) {
+                listed[atomicAdd(fb, 1ull)] = (int32_t)t;
+                continue;
+            }
             val = near_fp64(g1.type, g1.c, g1.n, g2.c, g2.v);
             atomicAdd(fb, 1ull);
         }
+        if (!isfinite(val)) atomicOr(status, 1u);
+        c32[l] = val;
+    }
+}
+
+__global__ void __launch_bounds__(64) k_fill_near_fp64(const unsigned long long *__restrict__ n_listed, const int32_t *__restrict__ listed,
+                                                       const int32_t *__restrict__ near_link, const int32_t *__restrict__ near_row,
+                                                       const uint32_t *__restrict__ src, const NodeGeo *__restrict__ geo,
+                                                       float *__restrict__ c32, unsigned *status) {
+    const int64_t n = (int64_t)*n_listed;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t t = listed[q];
+        const int64_t l = near_link[t];
+        const NodeGeo &g1 = geo[near_row[t]], &g2 = geo[src[l] & kSrcMask];
+        const float val = near_fp64(g1.type, g1.c, g1.n, g2.c, g2.v);
         if (!isfinite(val)) atomicOr(status, 1u);
         c32[l] = val;
     }
@@ -3913,7 +3941,7 @@ void problem_destroy(DeviceProblem *p) {
     dfree(p->geo); dfree(p->link_ptr); dfree(p->link_src); dfree(p->leaf_node); dfree(p->parent);
     dfree(p->left); dfree(p->right); dfree(p->node_lfirst); dfree(p->leaf_eb); dfree(p->leaf_ea); dfree(p->leaf_weight);
     dfree(p->coef64); dfree(p->coef32); dfree(p->self); dfree(p->rself); dfree(p->rself32); dfree(p->srself); dfree(p->status);
-    dfree(p->near_link); dfree(p->near_row); dfree(p->tri); dfree(p->quad); dfree(p->tri32); dfree(p->fill_fp64);
+    dfree(p->near_link); dfree(p->near_row); dfree(p->near_fp64); dfree(p->tri); dfree(p->quad); dfree(p->tri32); dfree(p->fill_fp64);
     SweepPlan &pl = p->plan;
     dfree(pl.blk_leaf_first); dfree(pl.blk_nleaves); dfree(pl.blk_lvl_first); dfree(pl.blk_nlvls); dfree(pl.blk_root);
     dfree(pl.lvl_ptr); dfree(pl.lvl_nodes); dfree(pl.lvl_kids); dfree(pl.blk_node_first); dfree(pl.blk_chain); dfree(pl.chain);
@@ -3958,7 +3986,7 @@ int64_t problem_estimate_bytes(const fcg_model_arrays &a, int precision, int rhs
     b += Np * (int64_t)(4 * 7 + 4 + 12 + 4 + 8);          // sweep plan: blocks, levels, children, top forest, chains (typical)
     b += L * (4 + c);                                                  // links
     b += Np * (4 + 8 * 4 + 4);                                         // leaf maps, permittivities, self terms, geometry map
-    b += L * 8 + Nn * (int64_t)(precision == FCG_PREC_FP64 ? sizeof(fcg_tri64) + sizeof(fcg_quad64) : sizeof(fcg_tri32));  // near list (bound) and tables
+    b += L * (precision == FCG_PREC_FP64 ? 8 : 12) + Nn * (int64_t)(precision == FCG_PREC_FP64 ? sizeof(fcg_tri64) + sizeof(fcg_quad64) : sizeof(fcg_tri32));  // near list (bound) and tables
     b += (int64_t)kp * Nn * (8 * 3 + 4 + 8);                           // matvec node work
     b += (int64_t)k * Np * 8 * (5 + vecs);                             // Krylov vectors and basis
     b += (int64_t)k * (steps + 1) * nch * 8;                           // partial sums
@@ -4054,10 +4082,22 @@ int problem_fill(DeviceProblem *p) {
         FCG_CK(cudaGetLastError());
         p->timings.launches++;
         if (p->n_near > 0) {
-            if (mixed)
-                k_fill_near32<<<grid_for(p->n_near, 128, sms), 128, 0, s>>>(p->n_near, p->near_link, p->near_row, p->link_src,
-                                                                           p->geo, p->tri32, p->coef32, p->status, p->fill_fp64);
-            else
+            if (mixed) {
+                const int grid = grid_for(p->n_near, 128, sms);
+                if (p->cond_cols.size() == (size_t)p->n_cond_all) {  // no dielectric panels
+                    int r;
+                    if (!p->near_fp64 && (r = dalloc(&p->near_fp64, (size_t)p->n_near, p->bytes)) != FCG_NORMAL_END) return r;
+                    k_fill_near32<true><<<grid, 128, 0, s>>>(p->n_near, p->near_link, p->near_row, p->link_src, p->geo, p->tri32,
+                                                             p->coef32, p->status, p->fill_fp64, p->near_fp64);
+                    // before k_fill_self32, which counts on in the same word
+                    k_fill_near_fp64<<<(int)std::min<int64_t>((p->n_near + 63) / 64, (int64_t)sms * 16), 64, 0, s>>>(
+                        p->fill_fp64, p->near_fp64, p->near_link, p->near_row, p->link_src, p->geo, p->coef32, p->status);
+                    p->timings.launches++;
+                } else {
+                    k_fill_near32<false><<<grid, 128, 0, s>>>(p->n_near, p->near_link, p->near_row, p->link_src, p->geo, p->tri32,
+                                                              p->coef32, p->status, p->fill_fp64, NULL);
+                }
+            } else
                 k_fill_near<<<grid_for(p->n_near, 128, sms), 128, 0, s>>>(p->n_near, p->near_link, p->near_row, p->link_src,
                                                                          p->geo, p->tri, p->coef64, p->coef32, p->status);
             FCG_CK(cudaGetLastError());
