@@ -75,31 +75,50 @@ void problem_cancel(DeviceProblem *p);
 // right-hand sides in at most `iterations` Arnoldi steps
 int64_t problem_estimate_bytes(const fcg_model_arrays &a, int precision, int rhs, int iterations);
 
+// Root pairs of the link traversal (element ids, two per pair, and the
+// recursion level each is visited at) and the node of every element, in host
+// or in device memory.
+struct LinkRoots {
+    int64_t n = 0;
+    std::shared_ptr<int32_t> pairs, node_of;
+    std::shared_ptr<uint16_t> level;
+};
+
 // Link construction on the device (csrc/link_build.cu): the traversal of
-// the element hierarchy `el` from the root pairs (root_a[i], root_b[i]),
-// visited at recursion level root_level[i], in the host builder's order;
-// node_of maps element ids to node ids. Fills link_ptr (n_nodes + 1) and
+// the element hierarchy `el` from the root pairs, in the host builder's order.
+// `el` and the roots' arrays are in device memory with on_device, else in host
+// memory. Fills link_ptr (n_nodes + 1) and
 // link_src exactly as the host traversal and its stable bucketing do, and
 // max_level with the deepest recursion level of the traversal. With
 // device_src the link sources stay in device memory (complete when the call
 // returns; freed with the last reference) and link_src is left empty.
 struct Element;
-int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const int32_t *root_a, const int32_t *root_b,
-                      const uint16_t *root_level, int64_t n_roots, const int32_t *node_of, int64_t n_nodes, double eps,
-                      double max_side, double max_area, std::vector<int64_t> &link_ptr, std::vector<int32_t> &link_src,
-                      int &max_level, std::string &err, std::shared_ptr<int32_t> *device_src = nullptr);
+int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const LinkRoots &roots, bool on_device,
+                      int64_t n_nodes, double eps, double max_side, double max_area, std::vector<int64_t> &link_ptr,
+                      std::vector<int32_t> &link_src, int &max_level, std::string &err,
+                      std::shared_ptr<int32_t> *device_src = nullptr);
 
 // Mesh refinement on the device (csrc/mesh_build.cu): the closure of the
 // refinement of the root pairs (root_a[i], root_b[i]) with root_meta[i] =
 // recursion level | kMeshSelfPair for pairs of the self pass. `el` (with
 // `depth`, every element's depth in its conductor's tree) is replaced by the
-// refined hierarchy; max_mesh_eps and max_level receive the largest weight of
-// an unrefined pair and the deepest pair level.
+// refined hierarchy, or, from keep_from elements on, left in device memory
+// (`kept`, n_kept elements; el is then empty); max_mesh_eps and max_level
+// receive the largest weight of an unrefined pair and the deepest pair level.
 constexpr uint16_t kMeshSelfPair = 0x8000;
 int mesh_refine_device(DeviceContext &ctx, std::vector<Element> &el, const std::vector<int32_t> &depth,
                        const std::vector<int32_t> &root_a, const std::vector<int32_t> &root_b,
                        const std::vector<uint16_t> &root_meta, double mesh_eps, double mesh_curv, double max_side,
-                       double max_area, double &max_mesh_eps, int &max_level, std::string &err);
+                       double max_area, int64_t keep_from, std::shared_ptr<Element> &kept, int64_t &n_kept,
+                       double &max_mesh_eps, int &max_level, std::string &err);
+
+// Flattening on the device (csrc/tree_flatten.cu) of the refined hierarchy
+// d_el (device memory): the node and leaf arrays of `M` as the host builder
+// fills them (the links aside; in device memory with keep_nodes), every conductor's leaf count, the link
+// traversal's root pairs (in device memory) and the depth of the deepest tree.
+struct Model;
+int tree_flatten_device(DeviceContext &ctx, const Element *d_el, int64_t ne, const std::vector<int32_t> &tops, bool keep_nodes,
+                        Model &M, std::vector<int64_t> &cond_leaves, LinkRoots &out, int &max_depth, std::string &err);
 
 // Super hierarchy on the device (csrc/super_build.cu): every conductor's
 // panels (element ids in `el`, conductors in solver order) split by the host

@@ -238,10 +238,10 @@ struct Level {
         }                                                                                            \
     } while (0)
 
-int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const int32_t *root_a, const int32_t *root_b,
-                      const uint16_t *root_level, int64_t n_roots, const int32_t *node_of, int64_t n_nodes, double eps,
-                      double max_side, double max_area, std::vector<int64_t> &link_ptr, std::vector<int32_t> &link_src,
-                      int &max_level, std::string &err, std::shared_ptr<int32_t> *device_src) {
+int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const LinkRoots &roots, bool on_device,
+                      int64_t n_nodes, double eps, double max_side, double max_area, std::vector<int64_t> &link_ptr,
+                      std::vector<int32_t> &link_src, int &max_level, std::string &err,
+                      std::shared_ptr<int32_t> *device_src) {
     LB_CK(cudaSetDevice(ctx.device));
     Bufs B;
     LB_CK(cudaStreamCreateWithFlags(&B.s, cudaStreamNonBlocking));
@@ -250,10 +250,11 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const i
     link_ptr.assign((size_t)n_nodes + 1, 0);
     link_src.clear();
     max_level = 0;
+    const int64_t n_roots = roots.n;
     if (n_roots == 0 || n_nodes == 0) return FCG_NORMAL_END;
 
-    Element *d_el;
-    int32_t *d_node_of;
+    const Element *d_el = el;
+    const int32_t *d_node_of = roots.node_of.get();
     long long *d_scalars;  // [0] scan total, [1] spare
     int *d_max_level;
     unsigned *d_bad;
@@ -263,13 +264,19 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const i
     const bool trace = getenv("FCG_TRACE") != nullptr;
     const auto t_begin = std::chrono::steady_clock::now();
     LB_CK(B.alloc(&d_count, kMaxGroup));
-    LB_CK(B.alloc(&d_el, (size_t)ne));
-    LB_CK(B.alloc(&d_node_of, (size_t)ne));
     LB_CK(B.alloc(&d_scalars, 2));
     LB_CK(B.alloc(&d_max_level, 1));
     LB_CK(B.alloc(&d_bad, 1));
-    LB_CK(cudaMemcpyAsync(d_el, el, (size_t)ne * sizeof(Element), cudaMemcpyHostToDevice, s));
-    LB_CK(cudaMemcpyAsync(d_node_of, node_of, (size_t)ne * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+    if (!on_device) {
+        Element *up;
+        int32_t *up_of;
+        LB_CK(B.alloc(&up, (size_t)ne));
+        LB_CK(B.alloc(&up_of, (size_t)ne));
+        LB_CK(cudaMemcpyAsync(up, el, (size_t)ne * sizeof(Element), cudaMemcpyHostToDevice, s));
+        LB_CK(cudaMemcpyAsync(up_of, d_node_of, (size_t)ne * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+        d_el = up;
+        d_node_of = up_of;
+    }
     LB_CK(cudaMemsetAsync(d_max_level, 0, sizeof(int), s));
     LB_CK(cudaMemsetAsync(d_bad, 0, sizeof(unsigned), s));
 
@@ -278,13 +285,12 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const i
     {
         Level &L0 = lv[0];
         L0.n = n_roots;
-        std::vector<int2> h((size_t)n_roots);
-        for (int64_t i = 0; i < n_roots; i++) h[(size_t)i] = make_int2(root_a[i], root_b[i]);
+        const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
         LB_CK(B.alloc(&L0.pairs, (size_t)n_roots));
         LB_CK(B.alloc(&L0.root_level, (size_t)n_roots));
         LB_CK(B.alloc(&L0.rank, (size_t)n_roots));
-        LB_CK(cudaMemcpyAsync(L0.pairs, h.data(), (size_t)n_roots * sizeof(int2), cudaMemcpyHostToDevice, s));
-        LB_CK(cudaMemcpyAsync(L0.root_level, root_level, (size_t)n_roots * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
+        LB_CK(cudaMemcpyAsync(L0.pairs, roots.pairs.get(), (size_t)n_roots * sizeof(int2), kind, s));
+        LB_CK(cudaMemcpyAsync(L0.root_level, roots.level.get(), (size_t)n_roots * sizeof(uint16_t), kind, s));
     }
 
     // frontier expansion, one level per launch. A level has at most twice the
@@ -474,10 +480,7 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const i
     }
     LB_CK(cudaMemcpyAsync(link_ptr.data(), d_ptr, ((size_t)n_nodes + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     if (device_src) {
-        // hand the sources over: off the builder's list, freed by the last owner
-        auto it = std::find(B.live.begin(), B.live.end(), (void *)d_src);
-        if (it != B.live.end()) B.live.erase(it);
-        device_src->reset(d_src, [](int32_t *q) { cudaFreeAsync(q, 0); });
+        *device_src = B.hand_over(d_src);
         link_src.clear();
     } else {
         link_src.resize((size_t)nent);

@@ -329,7 +329,8 @@ __global__ void __launch_bounds__(256) k_mesh_grow(LevelHead *__restrict__ head,
 int mesh_refine_device(DeviceContext &ctx, std::vector<Element> &el, const std::vector<int32_t> &depth,
                        const std::vector<int32_t> &root_a, const std::vector<int32_t> &root_b,
                        const std::vector<uint16_t> &root_meta, double mesh_eps, double mesh_curv, double max_side,
-                       double max_area, double &max_mesh_eps, int &max_level, std::string &err) {
+                       double max_area, int64_t keep_from, std::shared_ptr<Element> &kept, int64_t &n_kept,
+                       double &max_mesh_eps, int &max_level, std::string &err) {
     MB_CK(cudaSetDevice(ctx.device));
     Bufs B;
     MB_CK(cudaStreamCreateWithFlags(&B.s, cudaStreamNonBlocking));
@@ -490,9 +491,17 @@ int mesh_refine_device(DeviceContext &ctx, std::vector<Element> &el, const std::
     unsigned long long eps_bits = 0;
     MB_CK(cudaMemcpyAsync(&eps_bits, d_max_eps, sizeof(eps_bits), cudaMemcpyDeviceToHost, s));
     MB_CK(cudaMemcpyAsync(&max_level, d_max_level, sizeof(int), cudaMemcpyDeviceToHost, s));
-    el.resize((size_t)ne);
-    MB_CK(cudaMemcpyAsync(el.data(), d_el, (size_t)ne * sizeof(Element), cudaMemcpyDeviceToHost, s));
+    if (ne >= keep_from) {
+        el.clear();
+    } else {
+        el.resize((size_t)ne);
+        MB_CK(cudaMemcpyAsync(el.data(), d_el, (size_t)ne * sizeof(Element), cudaMemcpyDeviceToHost, s));
+    }
     MB_CK(cudaStreamSynchronize(s));
+    if (ne >= keep_from) {
+        kept = B.hand_over(d_el);
+        n_kept = ne;
+    }
     double me;
     memcpy(&me, &eps_bits, sizeof me);
     max_mesh_eps = me;

@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <memory>
 #include <vector>
 
 namespace fcg {
@@ -164,6 +165,14 @@ struct Bufs {
         if (it != live.end()) live.erase(it);
         cudaFreeAsync(p, s);
         p = nullptr;
+    }
+    // off the list: freed with the last reference (the stream's work on it is
+    // waited for before the allocator goes out of scope)
+    template <class T>
+    std::shared_ptr<T> hand_over(T *p) {
+        auto it = std::find(live.begin(), live.end(), (void *)p);
+        if (it != live.end()) live.erase(it);
+        return std::shared_ptr<T>(p, [](T *q) { cudaFreeAsync(q, 0); });
     }
 };
 

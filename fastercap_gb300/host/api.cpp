@@ -57,24 +57,25 @@ int fcg_model_build(const char *path, const fcg_build_options *opt, fcg_model **
 }  // extern "C"
 
 static int build_on(fcg::DeviceContext *dev, const char *path, const fcg_build_options *opt, bool links_on_device,
-                    fcg_model **out, char *err, size_t err_len);
+                    bool nodes_on_device, fcg_model **out, char *err, size_t err_len);
 
 namespace fcg {
-// a server job's model: built on the server's GPU with the link sources left
-// in device memory (problem creation copies them device to device)
-int model_build_device_links(DeviceContext *dev, const char *path, const fcg_build_options *opt, fcg_model **out, char *err,
-                             size_t err_len) {
-    return build_on(dev, path, opt, true, out, err, err_len);
+// a model built on the GPU with the link sources, and with nodes_too (a
+// server job's, which no host code reads) the node arrays, left in device
+// memory: problem creation copies them device to device
+int model_build_device_links(DeviceContext *dev, const char *path, const fcg_build_options *opt, bool nodes_too, fcg_model **out,
+                             char *err, size_t err_len) {
+    return build_on(dev, path, opt, true, nodes_too, out, err, err_len);
 }
 }  // namespace fcg
 
 extern "C" int fcg_model_build_on(fcg_context *ctx, const char *path, const fcg_build_options *opt, fcg_model **out,
                                   char *err, size_t err_len) {
-    return build_on(ctx ? ctx->dev : nullptr, path, opt, false, out, err, err_len);
+    return build_on(ctx ? ctx->dev : nullptr, path, opt, false, false, out, err, err_len);
 }
 
 static int build_on(fcg::DeviceContext *dev, const char *path, const fcg_build_options *opt, bool links_on_device,
-                    fcg_model **out, char *err, size_t err_len) {
+                    bool nodes_on_device, fcg_model **out, char *err, size_t err_len) {
     if (!path || !out) return FCG_GENERIC_ERROR;
     *out = NULL;
     fcg::BuildOptions o;
@@ -85,6 +86,7 @@ static int build_on(fcg::DeviceContext *dev, const char *path, const fcg_build_o
         o.verbose = opt->verbose != 0;
     }
     o.links_on_device = links_on_device && dev;
+    o.nodes_on_device = nodes_on_device && dev;
     fcg_model *fm = new (std::nothrow) fcg_model();
     if (!fm) return FCG_OUT_OF_MEMORY;
     std::string e;
@@ -146,6 +148,19 @@ int fcg_model_arrays_get(const fcg_model *fm, fcg_model_arrays *a) {
     a->link_ptr = m.link_ptr.data();
     a->link_src = m.d_link_src ? m.d_link_src.get() : m.link_src.data();
     a->leaf_diel = m.leaf_diel.data();
+    if (const fcg::DeviceNodes *d = m.d_nodes.get()) {
+        a->node_type = d->type;
+        a->node_left = d->left;
+        a->node_right = d->right;
+        a->node_leaf_first = d->leaf_first;
+        a->node_leaf_count = d->leaf_count;
+        a->node_vertices = d->vert;
+        a->node_centroid = d->cent;
+        a->node_normal = d->norm;
+        a->node_area = d->area;
+        a->node_maxside = d->maxside;
+        a->leaf_diel = d->leaf_diel;
+    }
     a->cond_is_diel = fm->cond_is_diel.data();
     a->cond_leaf_first = fm->cond_first.data();
     a->cond_leaf_count = fm->cond_count.data();
@@ -468,7 +483,7 @@ struct SolveRun {
 static int build_model_at(fcg_context *ctx, const CmdOptions &o, double mesh_eps, fcg_model **m, fcg_model_info &info) {
     fcg_build_options bo = {mesh_eps, o.eps_ratio, o.mesh_curv, o.verbose ? 1 : 0};
     char ebuf[512] = {0};
-    int r = fcg::model_build_device_links(ctx->dev, o.file.c_str(), &bo, m, ebuf, sizeof ebuf);
+    int r = fcg::model_build_device_links(ctx->dev, o.file.c_str(), &bo, false, m, ebuf, sizeof ebuf);
     if (r != FCG_NORMAL_END) { printf("Error: %s\n", ebuf); return r; }
     fcg_model_info_get(*m, &info);
     return FCG_NORMAL_END;

@@ -16,7 +16,7 @@ struct fcg_problem {
 namespace fcg {
 // fcg_model_build_on for a server job: the link sources stay in device
 // memory (the model's arrays then point there); host/api.cpp
-int model_build_device_links(DeviceContext *dev, const char *path, const fcg_build_options *opt, fcg_model **out, char *err,
+int model_build_device_links(DeviceContext *dev, const char *path, const fcg_build_options *opt, bool nodes_too, fcg_model **out, char *err,
                              size_t err_len);
 }  // namespace fcg
 

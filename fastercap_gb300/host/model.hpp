@@ -21,6 +21,10 @@ struct BuildOptions {
     // device builds only: leave the link sources in device memory
     // (Model::d_link_src) instead of copying them to link_src
     bool links_on_device = false;
+    // device builds only: leave the node and leaf arrays of a model flattened
+    // on the device there (Model::d_nodes); for models that only a problem
+    // creation reads
+    bool nodes_on_device = false;
 };
 
 // One element of the hierarchy: an input panel, a refined sub-panel or a
@@ -48,6 +52,16 @@ struct Conductor {
     int64_t leaf_count = 0;
 };
 
+// Node and leaf arrays in device memory
+struct DeviceNodes {
+    const uint8_t *type = nullptr, *leaf_diel = nullptr;
+    const int32_t *left = nullptr, *right = nullptr;
+    const int64_t *leaf_first = nullptr, *leaf_count = nullptr;
+    const float *vert = nullptr, *cent = nullptr, *norm = nullptr;
+    const double *area = nullptr, *maxside = nullptr;
+    std::vector<std::shared_ptr<const void>> owned;
+};
+
 // Flattened model (post-order node array, CSR links by destination node).
 struct Model {
     // nodes
@@ -64,6 +78,10 @@ struct Model {
     // the link sources in device memory when the build left them there
     // (BuildOptions::links_on_device); link_src is then empty
     std::shared_ptr<int32_t> d_link_src;
+    // the node and leaf arrays in device memory when the build left them there
+    // (BuildOptions::nodes_on_device); the vectors of the same names, cond,
+    // maxside_idx and leaf_node are then empty
+    std::unique_ptr<DeviceNodes> d_nodes;
     // leaves
     std::vector<int32_t> leaf_node;                // node of every leaf
     std::vector<uint8_t> leaf_diel;

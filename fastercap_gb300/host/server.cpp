@@ -97,7 +97,7 @@ static int count_conductors(const fcg_model_arrays &a) {
 static int build_file_job(fcg_server *s, Job *j) {
     double t0 = now_ms();
     char ebuf[512] = {0};
-    int r = fcg::model_build_device_links(s->ctx, j->path.c_str(), &j->bopt, &j->model, ebuf, sizeof ebuf);
+    int r = fcg::model_build_device_links(s->ctx, j->path.c_str(), &j->bopt, true, &j->model, ebuf, sizeof ebuf);
     j->build_ms = now_ms() - t0;
     if (r != FCG_NORMAL_END) {
         j->error = ebuf[0] ? std::string(ebuf) : fcg::get_error();
@@ -125,6 +125,11 @@ static void run_job(fcg_server *s, Job *j, void *stream) {
     int r = FCG_NORMAL_END;
     if (j->from_file) r = build_file_job(s, j);
     if (r == FCG_NORMAL_END) r = fcg::problem_create(*s->ctx, j->a, j->precision, stream, &p);
+    // the problem holds its own copies: the model's device memory goes back now
+    if (j->model) {
+        fcg_model_free(j->model);
+        j->model = nullptr;
+    }
     // a job solves once: measuring launch shapes would not pay
     if (r == FCG_NORMAL_END) fcg::problem_set_tuning(p, false);
     if (r == FCG_NORMAL_END) {
@@ -150,10 +155,6 @@ static void run_job(fcg_server *s, Job *j, void *stream) {
             j->prob = nullptr;
         }
         fcg::problem_destroy(p);
-    }
-    if (j->model) {
-        fcg_model_free(j->model);
-        j->model = nullptr;
     }
     j->status = r;
     if (r != FCG_NORMAL_END && j->error.empty()) j->error = fcg::get_error();
