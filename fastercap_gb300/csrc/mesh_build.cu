@@ -64,7 +64,7 @@ static_assert(sizeof(Element) == 96, "element record layout");
 // geometric normal (fcg_geo_normal) in FP32 and a bound on each component's
 // distance to the FP64 path's value; false when a super node's Newell modulus
 // is within rounding of the normalisation cut-off
-__device__ __forceinline__ bool geo_normal32(const Element &e, float &x, float &y, float &z, float &err) {
+__device__ __forceinline__ bool geo_normal32(const pair32::PairElement &e, float &x, float &y, float &z, float &err) {
     if (!(e.type & FCG_IS_SUPER_NODE)) {
         x = e.n[0]; y = e.n[1]; z = e.n[2];
         err = 0.0f;
@@ -72,6 +72,7 @@ __device__ __forceinline__ bool geo_normal32(const Element &e, float &x, float &
     }
     float n[3];
     n[0] = n[1] = n[2] = 0.0f;
+#pragma unroll
     for (int i = 0; i < 3; i++) {  // the float sums of fcg_newell_normal, same operations
         int j = i + 1 > 2 ? 0 : i + 1;
         const float *a = e.v + 3 * i, *b = e.v + 3 * j;
@@ -94,8 +95,8 @@ __device__ __forceinline__ bool geo_normal32(const Element &e, float &x, float &
 
 // fcg_mesh_decision in FP32: 1 / 2 refine (split the larger-area element),
 // 0 no refinement (c1, c2 and their bounds e1, e2 are the pair's weights),
-// -1 only the FP64 test can tell
-__device__ int mesh_decide32(const Element &A, const Element &B, bool selfc, float e, float mesh_curv, float inv_max_area,
+// -1 only the FP64 test can tell, -2 a near pair, left alone without `near`
+__device__ __forceinline__ int mesh_decide32(pair32::PairElement &A, pair32::PairElement &B, bool near, bool selfc, float e, float mesh_curv, float inv_max_area,
                              float inv_max_side, float &c1, float &e1, float &c2, float &e2) {
     using namespace pair32;
     float dx = A.c[0] - B.c[0], dy = A.c[1] - B.c[1], dz = A.c[2] - B.c[2];  // fcg_fsub's float values
@@ -104,6 +105,11 @@ __device__ int mesh_decide32(const Element &A, const Element &B, bool selfc, flo
     float rho = r / (float)rm;
     if (!(r > 1e-10f) || !(fabsf(rho - 2.0f) > 1e-5f)) return -1;
     bool quad = rho < 2.0f;
+    if (quad && !near) return -2;
+    if (quad || (selfc && ((A.type | B.type) & FCG_IS_SUPER_NODE))) {
+        A.vertices();
+        B.vertices();
+    }
     float cc = 1.0f, cc_err = 0.0f;
     if (selfc) {
         float ax, ay, az, ae, bx, by, bz, be;
@@ -176,20 +182,41 @@ __device__ __forceinline__ void emit_splits(LevelHead *head, int64_t ne, int f, 
 // is at least its lower bound), so only pairs near the running maximum take
 // the FP64 test for it. `lo_bits` holds that running lower bound (bits of a
 // non-negative double). With pre32 unset every pair takes the FP64 test.
-// A large level is bound by the gathers of its elements (96-byte records,
-// latency; four pairs a lane with one claim was slower, 218 -> 300 us a level
-// of 4M pairs), a small one by its launches: three kernels a level and a wait
-// for the host every few levels, instead of nine and one each: a 528-panel
-// model's refinement 1.74 -> 1.03 ms, its links 1.49 -> 0.90 ms.
+// A pair nearer than twice the larger side needs quadratures, some ten times
+// the instructions of a far one, and one such lane holds its warp: where a warp
+// has several rounds, near pairs wait in its queue until 32 of them run
+// together (one round: at once, the queue would only add a round). Levels of
+// 42 / 120 million pairs in all 2720 / 6335 -> 2063 / 4575 us with the 16-byte
+// loads of PairElement (without the queue 2420 / 5880, the queue alone 2435 /
+// 5320); a small level 11.7 -> 7.7. What is left is latency at 24 warps an SM:
+// 20 (no spills) 2277 / 5265, 32 2111 / 4504. Four pairs a lane with one claim
+// (218 -> 300 us a level of 4M pairs) and one claim a CTA (2842 / 7243) were
+// slower. A small level is bound by its launches: three kernels a level and a
+// wait for the host every few levels, instead of nine and one each: a 528-panel
+// model's refinement 1.74 -> 0.96 ms, its links 1.49 -> 0.90 ms.
 __global__ void __launch_bounds__(128, 6) k_mesh_level(LevelHead *__restrict__ head, const int2 *__restrict__ pairs,
                                                        const uint16_t *__restrict__ meta, Element *el, int *claim, int pre32, float e,
                                                        float mesh_curv, float inv_max_area, float inv_max_side, const LevelLists ls,
                                                        unsigned long long *lo_bits, int *max_level, unsigned *too_deep) {
-    const int64_t n = (int64_t)head->n, ne = (int64_t)head->ne;
+    __shared__ int32_t queue[4][64];
+    const int64_t n = (int64_t)head->n, ne = (int64_t)head->ne, stride = (int64_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
-    int lvl_max = 0;
-    // whole warps stay in the loop while their first pair exists (ballots below)
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i - lane < n; i += (int64_t)gridDim.x * blockDim.x) {
+    int32_t *q = queue[threadIdx.x >> 5];
+    const bool direct = n <= stride;  // a warp has one round at most
+    int lvl_max = 0, waiting = 0;
+    // whole warps stay in the loop (ballots below)
+    for (int64_t next = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);;) {
+        const bool near = waiting >= 32 || (waiting > 0 && next >= n);
+        if (!near && next >= n) break;
+        int64_t i = n;
+        if (near) {
+            const int take = min(waiting, 32);
+            waiting -= take;
+            if (lane < take) i = q[waiting + lane];
+        } else {
+            i = next + lane;
+            next += stride;
+        }
         int f = 0;
         bool leaf = false;
         double lo = 0.0;
@@ -203,9 +230,9 @@ __global__ void __launch_bounds__(128, 6) k_mesh_level(LevelHead *__restrict__ h
             if (lvl > kMaxMeshLevel) {
                 atomicOr(too_deep, 1u);
             } else if (pre32) {
-                const Element &A = el[pr.x], &B = el[pr.y];
+                pair32::PairElement A(el[pr.x]), B(el[pr.y]);
                 float c1 = 0, e1 = 0, c2 = 0, e2 = 0;
-                f = mesh_decide32(A, B, (m & kSelfBit) != 0, e, mesh_curv, inv_max_area, inv_max_side, c1, e1, c2, e2);
+                f = mesh_decide32(A, B, near || direct, (m & kSelfBit) != 0, e, mesh_curv, inv_max_area, inv_max_side, c1, e1, c2, e2);
                 leaf = ((f == 1 ? A.type : B.type) & FCG_IS_LEAF) != 0;
                 if (f == 0) {
                     // a kept pair: may its exact weight be the model's largest?
@@ -222,10 +249,14 @@ __global__ void __launch_bounds__(128, 6) k_mesh_level(LevelHead *__restrict__ h
                 f = -1;
             }
         }
-        const unsigned listed = __ballot_sync(0xffffffffu, f < 0);
+        const unsigned later = __ballot_sync(0xffffffffu, f == -2);  // none in a round from the queue
+        if (f == -2) q[waiting + __popc(later & ((1u << lane) - 1u))] = (int32_t)i;
+        waiting += __popc(later);
+        __syncwarp();
+        const unsigned listed = __ballot_sync(0xffffffffu, f == -1);
         if (listed) {
             const int64_t at = warp_claim(&head->n_listed, __popc(listed)) + __popc(listed & ((1u << lane) - 1u));
-            if (f < 0) ls.listed[at] = (int32_t)i;
+            if (f == -1) ls.listed[at] = (int32_t)i;
             for (int o = 16; o > 0; o >>= 1) lo = fmax(lo, __shfl_xor_sync(0xffffffffu, lo, o));
             if (lane == 0 && lo > 0.0) atomicMax(lo_bits, (unsigned long long)__double_as_longlong(lo));
         }

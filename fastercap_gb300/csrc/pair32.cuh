@@ -12,6 +12,8 @@
 #ifndef FCG_PAIR32_CUH
 #define FCG_PAIR32_CUH
 
+#include <stddef.h>
+
 #include "fc_potential.h"
 #include "../host/model.hpp"
 
@@ -19,6 +21,35 @@ namespace fcg {
 namespace pair32 {
 
 constexpr float kU = 5.9604645e-8f;  // 2^-24, unit roundoff of float
+
+// What a pre-test reads of an element, in registers by 16-byte loads (4 an
+// element, with the vertices, where a test needs them, 6; by fields 9 and 20).
+// The mesh levels gain by it (their comment has the figures); the link levels,
+// whose pairs are fewer and nearer, do not (744 -> 813 us in all) and read fields.
+struct PairElement {
+    float v[9], c[3], n[3];
+    double area, maxside;
+    unsigned type;
+    const float4 *rec;
+    __device__ __forceinline__ explicit PairElement(const Element &e) : rec(reinterpret_cast<const float4 *>(&e)) {
+        static_assert(sizeof(Element) == 96 && offsetof(Element, c) == 36 && offsetof(Element, n) == 48 &&
+                          offsetof(Element, area) == 64 && offsetof(Element, maxside) == 72 && offsetof(Element, type) == 88,
+                      "element record layout");
+        const float4 a = rec[2], b = rec[3];
+        const double2 d = reinterpret_cast<const double2 *>(rec)[4];
+        v[8] = a.x;
+        c[0] = a.y; c[1] = a.z; c[2] = a.w;
+        n[0] = b.x; n[1] = b.y; n[2] = b.z;
+        area = d.x;
+        maxside = d.y;
+        type = reinterpret_cast<const uint32_t *>(rec)[22] & 255u;
+    }
+    __device__ __forceinline__ void vertices() {
+        const float4 a = rec[0], b = rec[1];
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+};
 
 // unit normal of a dielectric evaluation element (fcg_diel_normal in FP32);
 // false when a super node's normal is within rounding of the 1e-12 cut-off
@@ -100,7 +131,8 @@ __device__ __forceinline__ bool quad2_32(float dx, float dy, float dz, const flo
 
 // one direction of CAutoRefine::RefineCriteria in FP32: the weight of source
 // S seen from evaluation element E (d = E.c - S.c), with its error bound
-__device__ __forceinline__ bool weight32(const Element &E, const Element &S, float dx, float dy, float dz, float r, bool quad,
+template <class EL>
+__device__ __forceinline__ bool weight32(const EL &E, const EL &S, float dx, float dy, float dz, float r, bool quad,
                                          float inv_max_area, float inv_max_side, float &cw, float &err) {
     bool diel = (E.type & FCG_IS_DIEL) != 0;
     float nx = 0.0f, ny = 0.0f, nz = 0.0f;
