@@ -481,11 +481,11 @@ int mesh_refine_device(DeviceContext &ctx, std::vector<Element> &el, const std::
                                                               max_side, max_area, ls, d_max_eps);
             int64_t next_bound = 3 * bound, grow = 2 * bound;
             if (next_bound > kNoWait) {
-                LevelHead h;
                 unsigned deep = 0;
-                MB_CK(cudaMemcpyAsync(&h, head, sizeof h, cudaMemcpyDeviceToHost, s));
+                MB_CK(cudaMemcpyAsync(heads.data(), d_head, (size_t)(g + 1) * sizeof(LevelHead), cudaMemcpyDeviceToHost, s));
                 MB_CK(cudaMemcpyAsync(&deep, d_too_deep, sizeof deep, cudaMemcpyDeviceToHost, s));
                 MB_CK(cudaStreamSynchronize(s));
+                const LevelHead &h = heads[(size_t)g];
                 waited = true;
                 next_bound = (int64_t)(2 * h.n_split + h.n_leaves);
                 grow = (int64_t)(2 * h.n_leaves);
@@ -507,13 +507,20 @@ int mesh_refine_device(DeviceContext &ctx, std::vector<Element> &el, const std::
             g++;
         } while (!waited && bound <= kNoWait && g < kMaxGroup);
         heads.resize((size_t)g + 1);
-        unsigned deep = 0;
-        MB_CK(cudaMemcpyAsync(heads.data(), d_head, heads.size() * sizeof(LevelHead), cudaMemcpyDeviceToHost, s));
-        MB_CK(cudaMemcpyAsync(&deep, d_too_deep, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-        MB_CK(cudaStreamSynchronize(s));
-        if (deep) {
-            err = "mesh refinement recursion too deep (touching or overlapping panels?)";
-            return FCG_GENERIC_ERROR;
+        if (waited) {
+            // the last level's counts are known, and with them the next's size: one
+            // wait a level, not two (180 thousand elements 5.4 -> 4.2 ms)
+            heads.back().n = (unsigned long long)bound;
+            heads.back().ne = (unsigned long long)ne_bound;
+        } else {
+            unsigned deep = 0;
+            MB_CK(cudaMemcpyAsync(heads.data(), d_head, heads.size() * sizeof(LevelHead), cudaMemcpyDeviceToHost, s));
+            MB_CK(cudaMemcpyAsync(&deep, d_too_deep, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+            MB_CK(cudaStreamSynchronize(s));
+            if (deep) {
+                err = "mesh refinement recursion too deep (touching or overlapping panels?)";
+                return FCG_GENERIC_ERROR;
+            }
         }
         for (size_t q = 0; q + 1 < heads.size(); q++) tests += (long long)heads[q].n;
         n = (int64_t)heads.back().n;
