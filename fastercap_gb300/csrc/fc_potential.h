@@ -697,31 +697,40 @@ FCG_HD void fcg_pair_span(const E &A, const E &B, fcg_d3 *dist, double *rdist, d
 // for a dielectric evaluation element; rule-2 quadrature when the centroids
 // are closer than twice the larger side, the point formula beyond), weighted
 // by the source's area (and longest side, for a dielectric) relative to the
-// model's largest. True when either weight exceeds `e`.
+// model's largest. fcg_one_way: the weight of source B seen from A
+// (dist = A - B); fcg_refine_criteria: true when either weight exceeds `e`.
+template <class E>
+FCG_HD double fcg_one_way(const E &A, const E &B, fcg_d3 dist, double rdist, double rmax, double ccoeff, double max_side,
+                          double max_area) {
+    fcg_d3 n = fcg_diel_normal(A.type, A.n);
+    double pe;
+    bool diel = (A.type & FCG_IS_DIEL) != 0;
+    if (rdist / rmax < 2.0) {
+        fcg_d3 ca = fcg_widen(A.c);
+        pe = diel ? fcg_enfield_numerical(ca, B.v, n, 2) : fcg_potential_numerical(ca, B.v, 2);
+    } else {
+        if (diel) pe = (dist.x * n.x + dist.y * n.y + dist.z * n.z) / (rdist * rdist * rdist);
+        else pe = 1.0 / rdist;
+    }
+    if (diel) return fabs(pe * B.area * B.maxside / (max_side * max_area * ccoeff));
+    return fabs(pe * B.area / (max_area * ccoeff));
+}
+
 template <class E>
 FCG_HD bool fcg_refine_criteria(const E &A, const E &B, fcg_d3 dist, double rdist, double rmax, double e, double ccoeff,
                                 double max_side, double max_area, double *c1, double *c2) {
-    bool force = false;
-    fcg_d3 n1 = fcg_diel_normal(A.type, A.n), n2 = fcg_diel_normal(B.type, B.n);
-    double pe1, pe2;
-    bool d1 = (A.type & FCG_IS_DIEL) != 0, d2 = (B.type & FCG_IS_DIEL) != 0;
-    if (rdist / rmax < 2.0) {
-        fcg_d3 ca = fcg_widen(A.c), cb = fcg_widen(B.c);
-        pe1 = d1 ? fcg_enfield_numerical(ca, B.v, n1, 2) : fcg_potential_numerical(ca, B.v, 2);
-        pe2 = d2 ? fcg_enfield_numerical(cb, A.v, n2, 2) : fcg_potential_numerical(cb, A.v, 2);
-    } else {
-        if (d1) pe1 = (dist.x * n1.x + dist.y * n1.y + dist.z * n1.z) / (rdist * rdist * rdist);
-        else pe1 = 1.0 / rdist;
-        if (d2) pe2 = (-dist.x * n2.x + -dist.y * n2.y + -dist.z * n2.z) / (rdist * rdist * rdist);
-        else pe2 = 1.0 / rdist;
-    }
-    if (d1) *c1 = fabs(pe1 * B.area * B.maxside / (max_side * max_area * ccoeff));
-    else *c1 = fabs(pe1 * B.area / (max_area * ccoeff));
-    if (*c1 > e) force = true;
-    if (d2) *c2 = fabs(pe2 * A.area * A.maxside / (max_side * max_area * ccoeff));
-    else *c2 = fabs(pe2 * A.area / (max_area * ccoeff));
-    if (*c2 > e) force = true;
-    return force;
+    *c1 = fcg_one_way(A, B, dist, rdist, rmax, ccoeff, max_side, max_area);
+    *c2 = fcg_one_way(B, A, fcg_mk(-dist.x, -dist.y, -dist.z), rdist, rmax, ccoeff, max_side, max_area);
+    return *c1 > e || *c2 > e;
+}
+
+// the side a pair that needs refining recurses into (not both leaves)
+template <class E>
+FCG_HD int fcg_link_side(const E &A, const E &B) {
+    bool leaf1 = (A.type & FCG_IS_LEAF) != 0, leaf2 = (B.type & FCG_IS_LEAF) != 0;
+    if (!leaf1 && leaf2) return 1;
+    if (leaf1 && !leaf2) return 2;
+    return A.area > B.area ? 1 : 2;
 }
 
 // One step of CAutoRefine::RefineMutual (Solver/Autorefine.cpp:3096-3235):
@@ -737,9 +746,7 @@ FCG_HD int fcg_link_decision(const E &A, const E &B, double eps, double max_side
     double rdist, rmax, c1, c2;
     fcg_pair_span(A, B, &dist, &rdist, &rmax);
     if (!fcg_refine_criteria(A, B, dist, rdist, rmax, eps, 1.0, max_side, max_area, &c1, &c2)) return 0;
-    if (!leaf1 && leaf2) return 1;
-    if (leaf1 && !leaf2) return 2;
-    return A.area > B.area ? 1 : 2;
+    return fcg_link_side(A, B);
 }
 
 // ---------------------------------------------------------------- mesh
@@ -925,6 +932,12 @@ FCG_HD void fcg_subdivide(const E &P, E &Lc, E &Rc) {
     fcg_max_side3(Rc, rsl[0], rsl[1], rsl[2]);
 }
 
+template <class E>
+FCG_HD double fcg_curv_coeff(const E &A, const E &B, bool selfc, double mesh_curv) {
+    if (!selfc) return 1.0;
+    return (mesh_curv - 1.0) * (fcg_dot(fcg_geo_normal(A), fcg_geo_normal(B)) + 1.0) + 1.0;
+}
+
 // One step of CAutoRefine::DiscretizeMutual (Solver/Autorefine.cpp:2638-2730):
 // 0 = the pair is fine enough (c1, c2 hold its weights); 1 / 2 = refine by
 // splitting the larger-area element (B on ties). For sibling pairs
@@ -936,9 +949,7 @@ FCG_HD int fcg_mesh_decision(const E &A, const E &B, bool selfc, double e, doubl
     fcg_d3 dist;
     double rdist, rmax;
     fcg_pair_span(A, B, &dist, &rdist, &rmax);
-    double ccoeff;
-    if (selfc) ccoeff = (mesh_curv - 1.0) * (fcg_dot(fcg_geo_normal(A), fcg_geo_normal(B)) + 1.0) + 1.0;
-    else ccoeff = 1.0;
+    const double ccoeff = fcg_curv_coeff(A, B, selfc, mesh_curv);
     if (!fcg_refine_criteria(A, B, dist, rdist, rmax, e, ccoeff, max_side, max_area, c1, c2)) return 0;
     return A.area > B.area ? 1 : 2;
 }

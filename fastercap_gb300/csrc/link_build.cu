@@ -152,23 +152,38 @@ __global__ void __launch_bounds__(128) k_link_level(int64_t n0, const LevelCount
     if (lane == 0 && lvl) atomicMax(max_level, lvl);
 }
 
-// the FP64 test (the host builder's own code) for the level's listed pairs
+// The FP64 test (the host builder's own code) for the level's listed pairs: two
+// lanes a pair, one for each direction's weight, whose arithmetic does not
+// change when the two elements swap places (7.8 -> 5.2 us a level of a small
+// model; 25 levels of 10.8 million pairs 457 -> 278, 27 of 28 million 618 -> 370).
 __global__ void __launch_bounds__(128) k_link_level64(const int2 *__restrict__ pairs, const uint16_t *__restrict__ root_level, int64_t ne,
                                                       const Element *__restrict__ el, double eps, double max_side, double max_area,
                                                       int32_t *__restrict__ rank, int64_t next_cap, int2 *__restrict__ next,
                                                       uint16_t *__restrict__ next_level, LevelCount *count,
                                                       const int32_t *__restrict__ listed, unsigned *bad) {
     const int64_t m = (int64_t)count->listed;
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j - (threadIdx.x & 31) < m; j += (int64_t)gridDim.x * blockDim.x) {
+    const int odd = threadIdx.x & 1;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t - (threadIdx.x & 31) < 2 * m; t += (int64_t)gridDim.x * blockDim.x) {
         int f = -1;
         int64_t i = 0;
         int2 pr = make_int2(0, 0);
         uint16_t rl = 0;
-        if (j < m) {
-            i = listed[j];
+        double c = 0.0;
+        if (t < 2 * m) {
+            i = listed[t >> 1];
             pr = pairs[i];
             rl = root_level[i];
-            f = fcg_link_decision(el[pr.x], el[pr.y], eps, max_side, max_area);
+            const Element &A = el[odd ? pr.y : pr.x], &B = el[odd ? pr.x : pr.y];
+            fcg_d3 dist;
+            double rdist, rmax;
+            fcg_pair_span(A, B, &dist, &rdist, &rmax);
+            c = fcg_one_way(A, B, dist, rdist, rmax, 1.0, max_side, max_area);
+        }
+        const double c2 = __shfl_xor_sync(0xffffffffu, c, 1);
+        if (t < 2 * m && !odd) {
+            const Element &A = el[pr.x], &B = el[pr.y];
+            const bool link = (A.type & B.type & FCG_IS_LEAF) || !(c > eps || c2 > eps);
+            f = link ? 0 : fcg_link_side(A, B);
         }
         emit_children(count, ne, i, f, pr, rl, el, rank, next_cap, next, next_level, bad);
     }
