@@ -2799,21 +2799,43 @@ __global__ void k_refine_count(int S, const double *__restrict__ nr2, const doub
 // column from the last, the lane that owns z_i divides it by R_ii, then the
 // lanes update z_j -= R_ji z_i for all j < i at once (every z_j sees the
 // same sequence of updates as in a serial column-oriented sweep)
-__global__ void k_backsub(int S, int M, double *const *__restrict__ Hc, const double *g, const int *iters, double *z) {
+// A warp's chain of divisions is what it waits for: up to kBacksubShared
+// unknowns stay in shared memory, and the next column's address, diagonal and
+// first 32 entries are loaded ahead of the division they follow.
+// 4 solves of 35 steps 36 -> 19 us, 22 of 53 75 -> 36.
+// Longer cycles than kBacksubShared work in z itself: rare, and their columns
+// are then the time.
+constexpr int kBacksubShared = 512;
+__global__ void __launch_bounds__(128) k_backsub(int S, int M, double *const *__restrict__ Hc, const double *__restrict__ g,
+                                                 const int *__restrict__ iters, double *z) {
+    __shared__ double sh[4][kBacksubShared];
     const int sidx = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (sidx >= S) return;
     const int it = iters[sidx];
     double *zz = z + (int64_t)sidx * (M + 2);
     const double *gg = g + (int64_t)sidx * (M + 2);
-    for (int i = lane; i <= it; i += 32) zz[i] = gg[i];
+    const bool shared = it < kBacksubShared;
+    double *x = shared ? sh[threadIdx.x >> 5] : zz;
+    for (int i = lane; i <= it; i += 32) x[i] = gg[i];
     __syncwarp();
+    auto column = [&](int i) { return Hc[i] + (int64_t)sidx * (i + 2); };
+    const double *hc = it >= 0 ? column(it) : NULL;
+    double diag = it >= 0 ? hc[it] : 1.0, h0 = lane < it ? hc[lane] : 0.0;
     for (int i = it; i >= 0; i--) {
-        const double *hc = Hc[i] + (int64_t)sidx * (i + 2);
-        const double zi = zz[i] / hc[i];
-        for (int j = lane; j < i; j += 32) zz[j] = zz[j] - hc[j] * zi;
-        if (lane == 0) zz[i] = zi;
+        const double *next = i > 0 ? column(i - 1) : hc;
+        const double next_diag = i > 0 ? next[i - 1] : 1.0, next_h0 = lane < i - 1 ? next[lane] : 0.0;
+        const double zi = x[i] / diag;
+        if (lane < i) x[lane] = x[lane] - h0 * zi;
+        for (int j = lane + 32; j < i; j += 32) x[j] = x[j] - hc[j] * zi;
         __syncwarp();
+        if (lane == 0) x[i] = zi;
+        hc = next;
+        diag = next_diag;
+        h0 = next_h0;
     }
+    __syncwarp();
+    if (shared)
+        for (int i = lane; i <= it; i += 32) zz[i] = x[i];
 }
 
 // y[r][j] = sum_{jv <= iters(s)} z_s[jv] V_jv[r][j] (in pair arithmetic on
