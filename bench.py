@@ -829,10 +829,11 @@ def run_serving(args, rank, world, local_rank):
         "server": {"max_running": st["max_running"], "peak_in_use_bytes": st["peak_in_use"], "budget_bytes": st["budget"]},
         "e2e": {"value": mixed_top["solves_s"], "unit": "solves/s",
                 "h2d_bytes_per_step": int(np.mean([os.path.getsize(p) for p in paths])) + int(
-                    np.mean(panels) * 2 * 101 + np.mean(links) * 4),
+                    np.mean(panels) * 2 * 8),
                 "d2h_bytes_per_step": int(np.mean([c.nbytes for c in caps[("mixed", rates[-1])]])),
                 "note": "requests arrive as input files on the host; a request's time includes its model build, "
-                        "upload and the matrix read back (H2D counts the model arrays problem creation uploads)"},
+                        "upload and the matrix read back (H2D counts the input file and the row offsets: elements, nodes "
+                        "and links are made on the device and stay there)"},
         "gpu_launches": launches,
         "roofline": roof,
         "clocks": clk_summary,
