@@ -626,12 +626,18 @@ __device__ __forceinline__ void far_link64(int64_t l, int row, const uint32_t *_
     const bool diel = g1.type & FCG_IS_DIEL;
     fcg_d3 n = fcg_mk(0, 0, 0);
     if (diel) n = fcg_diel_normal(g1.type, g1.n);
-    double sum = 0.0, scale = (1.0 / FCG_FOUR_PI_TIMES_E0) / NP;
+    // 1 / (4 pi eps0 NP), rounded once: it enters every coefficient alike, so its
+    // rounding does not average out (formed as (1 / 4 pi eps0) / NP, and times
+    // fac before the sum, the potentials were 1.3 units of 2^-53 too large on
+    // average; so they are within 0.15, the reference's order of operations 0.2)
+    constexpr double kScale = NP == 1 ? 0x1.0bd99415ffcaep+33 : (NP == 3 ? 0x1.65221ac7ffb92p+31 : 0x1.65221ac7ffb92p+30);
+    double sum = 0.0, val;
     if constexpr (NP == 1) {
         const NodeGeo &g2 = geo[w & kSrcMask];
         const double dx = f2d_bits(g1.c[0] - g2.c[0]), dy = f2d_bits(g1.c[1] - g2.c[1]), dz = f2d_bits(g1.c[2] - g2.c[2]);
         const double ir = rsqrt64(dx * dx + dy * dy + dz * dz);
         sum = diel ? (dx * n.x + dy * n.y + dz * n.z) * (ir * ir * ir) : ir;
+        val = sum * kScale;
     } else {
         const fcg_quad64 &q = quad[w & kSrcMask];
         const double ax = q.a[0], ay = q.a[1], az = q.a[2], bx = q.b[0], by = q.b[1], bz = q.b[2];
@@ -653,9 +659,8 @@ __device__ __forceinline__ void far_link64(int64_t l, int row, const uint32_t *_
             const double ir = rsqrt64(dx * dx + dy * dy + dz * dz);
             sum += diel ? (dx * n.x + dy * n.y + dz * n.z) * (ir * ir * ir) : ir;
         }
-        scale *= q.fac;
+        val = sum * q.fac * kScale;
     }
-    const double val = sum * scale;
     if (!isfinite(val)) atomicOr(status, 1u);
     c64[l] = val;
 }
