@@ -4195,9 +4195,9 @@ int problem_get_coefficients(DeviceProblem *p, double *link_coef, double *self_c
 // (the mixed multi-right-hand-side link product moves four per 16-byte
 // gather); FP64 up to ten, where a lane owns two columns and every padding
 // column costs its share of the FP64 pipe, an even number
-static int kpad(int k) { return k <= 2 ? k : (k + 3) / 4 * 4; }
 static int kpad(const DeviceProblem *p, int k) {
-    return p->precision == FCG_PREC_FP64 && k <= 10 ? (k == 1 ? 1 : (k + 1) / 2 * 2) : kpad(k);
+    if (k <= 2) return k;
+    return p->precision == FCG_PREC_FP64 && k <= 10 ? (k + 1) / 2 * 2 : (k + 3) / 4 * 4;
 }
 
 static int ensure_matvec_ws(DeviceProblem *p, int kp) {
@@ -5498,7 +5498,7 @@ static size_t noalloc_need(const DeviceProblem *p, int kp) {
 int problem_matvec_noalloc(DeviceProblem *p, const double *d_q, double *d_v, int k) {
     if (!p->filled) { set_error("coefficients not filled"); return FCG_GENERIC_ERROR; }
     if (k < 1 || k > kMaxK) { set_error("right-hand sides per matvec must be in [1, 32]"); return FCG_GENERIC_ERROR; }
-    int kp = kpad(k);
+    int kp = kpad(p, k);
     size_t need = noalloc_need(p, kp);
     if (need > kNoAllocScratchBytes) {
         set_error("no-allocation matvec: the model needs " + std::to_string(need) + " bytes of node scratch for " +
