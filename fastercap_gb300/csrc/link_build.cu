@@ -231,9 +231,16 @@ __global__ void k_entries(int64_t P, const int2 *__restrict__ pairs, const int32
 // ------------------------------------------------------------------ host side
 constexpr size_t kMaxGroup = 24;       // levels launched at a time (the bound doubles: at most 18)
 constexpr int64_t kNoWait = 1 << 18;  // pairs up to which levels are launched without knowing their size
+// Pairs of room that the levels held may have beyond their sizes: a level is
+// made for twice the pairs of the one before, and about half of them split. Up to
+// this much (32 MB) it stays; then levels are copied to arrays of their sizes,
+// since all of them are held until the placement, whose counts and emitted
+// pairs (12 bytes a pair test, next to 12 of the levels) are the peak of the
+// build (127 million pair tests: 4745 -> 3159 MB).
+constexpr int64_t kUnusedPairs = 4 << 20;
 
 struct Level {
-    int64_t n = 0;
+    int64_t n = 0, room = 0, rank_room = 0;  // pairs, and what `pairs` and `rank` have room for
     int2 *pairs = nullptr;
     uint16_t *root_level = nullptr;
     int32_t *rank = nullptr;
@@ -301,9 +308,9 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const L
         Level &L0 = lv[0];
         L0.n = n_roots;
         const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+        L0.room = n_roots;
         LB_CK(B.alloc(&L0.pairs, (size_t)n_roots));
         LB_CK(B.alloc(&L0.root_level, (size_t)n_roots));
-        LB_CK(B.alloc(&L0.rank, (size_t)n_roots));
         LB_CK(cudaMemcpyAsync(L0.pairs, roots.pairs.get(), (size_t)n_roots * sizeof(int2), kind, s));
         LB_CK(cudaMemcpyAsync(L0.root_level, roots.level.get(), (size_t)n_roots * sizeof(uint16_t), kind, s));
     }
@@ -312,6 +319,16 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const L
     // pairs of the one before: the host waits for the counts only when that
     // bound has grown past kNoWait pairs since it last knew them.
     long long n_tests = 0, n_fp64 = 0;
+    // an array of n elements in the place of a larger one
+    auto shrink = [&](auto *&p, int64_t &room, int64_t n) -> cudaError_t {
+        if (room <= n) return cudaSuccess;
+        room = n;
+        auto *old = p;
+        cudaError_t e = B.alloc(&p, (size_t)n);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(p, old, (size_t)n * sizeof(*p), cudaMemcpyDeviceToDevice, s);
+        B.release(old);
+        return e;
+    };
     for (bool more = true; more;) {
         const size_t first = lv.size() - 1;  // its size is known
         int64_t bound = lv[first].n;
@@ -327,11 +344,12 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const L
                 listed_room = std::max<int64_t>(bound, kNoWait);
                 LB_CK(B.alloc(&d_listed, (size_t)listed_room));
             }
+            lv[d].rank_room = bound;
+            LB_CK(B.alloc(&lv[d].rank, (size_t)bound));
             Level nx;
-            nx.n = 2 * bound;
+            nx.n = nx.room = 2 * bound;
             LB_CK(B.alloc(&nx.pairs, (size_t)nx.n));
             LB_CK(B.alloc(&nx.root_level, (size_t)nx.n));
-            LB_CK(B.alloc(&nx.rank, (size_t)nx.n));
             const Level &L = lv[d];
             LevelCount *count = d_count + (d - first);
             k_link_level<<<grid_stride(bound, sms, 128), 128, 0, s>>>(
@@ -368,7 +386,18 @@ int link_build_device(DeviceContext &ctx, const Element *el, int64_t ne, const L
                 break;
             }
         }
+        // the levels with the most unused room first: each costs an allocation and a copy
+        int64_t unused = 0;
+        for (const Level &L : lv) unused += L.room - L.n;
+        for (int64_t least = kUnusedPairs / 16; unused > kUnusedPairs; least = 1)
+            for (Level &L : lv) {
+                if (L.room - L.n < least) continue;
+                unused -= L.room - L.n;
+                LB_CK(shrink(L.pairs, L.room, L.n));
+                LB_CK(shrink(L.rank, L.rank_room, L.n));
+            }
     }
+    B.release(d_listed);
     unsigned bad = 0;
     LB_CK(cudaMemcpyAsync(&bad, d_bad, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     LB_CK(cudaMemcpyAsync(&max_level, d_max_level, sizeof(int), cudaMemcpyDeviceToHost, s));
