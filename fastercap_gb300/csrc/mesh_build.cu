@@ -546,6 +546,23 @@ int mesh_refine_device(DeviceContext &ctx, std::vector<Element> &el, const std::
     MB_CK(cudaMemcpyAsync(&max_level, d_max_level, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (ne >= keep_from) {
         el.clear();
+        // to its size: the room for growth, at least 2^20 elements, would stay
+        // through the flattening and the links, whose memory is the build's peak
+        for (int f = 0; f < 2; f++) {
+            B.release(pairs[f]);
+            B.release(meta[f]);
+        }
+        B.release(ls.split_pairs);
+        B.release(ls.split_meta);
+        B.release(ls.leaves);
+        B.release(ls.listed);
+        B.release(d_depth);
+        B.release(d_claim);
+        Element *fit;
+        MB_CK(B.alloc(&fit, (size_t)ne));
+        MB_CK(cudaMemcpyAsync(fit, d_el, (size_t)ne * sizeof(Element), cudaMemcpyDeviceToDevice, s));
+        B.release(d_el);
+        d_el = fit;
     } else {
         el.resize((size_t)ne);
         MB_CK(cudaMemcpyAsync(el.data(), d_el, (size_t)ne * sizeof(Element), cudaMemcpyDeviceToHost, s));

@@ -54,3 +54,12 @@ def test_traversal(tmp_path, mesh, eps_ratio):
     # and the elements' arrays, which grow by 2^20 elements or to twice their size
     elements = 96 * max(2 * nodes, nodes + (1 << 20))
     assert peak <= 24 * tests + (48 << 20) + 300 * nodes + elements
+
+
+@pytest.mark.parametrize("mesh,eps_ratio", [(1e-3, 1.0), (6e-4, 1.0), (1e-3, 0.2)])
+def test_elements_beside_the_links(tmp_path, mesh, eps_ratio):
+    """the refined elements' room for growth (100 MB and more) is gone by then"""
+    path = str(tmp_path / "in.txt")
+    geo.Crossing(k=8, length=30.0, pitch=3.0, gap=1.0).write(path)
+    peak, tests, nodes = build_peak(path, mesh_eps=mesh, eps_ratio=eps_ratio)
+    assert peak <= 24 * tests + (48 << 20) + 300 * nodes
