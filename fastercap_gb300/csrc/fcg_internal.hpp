@@ -119,6 +119,8 @@ int mesh_refine_device(DeviceContext &ctx, std::vector<Element> &el, const std::
 struct Model;
 int tree_flatten_device(DeviceContext &ctx, const Element *d_el, int64_t ne, const std::vector<int32_t> &tops, bool keep_nodes,
                         Model &M, std::vector<int64_t> &cond_leaves, LinkRoots &out, int &max_depth, std::string &err);
+// The arrays of M.d_nodes into the model's vectors; the device memory goes back.
+int tree_nodes_to_host(DeviceContext &ctx, Model &M, std::string &err);
 
 // Super hierarchy on the device (csrc/super_build.cu): every conductor's
 // panels (element ids in `el`, conductors in solver order) split by the host

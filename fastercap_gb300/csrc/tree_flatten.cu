@@ -308,4 +308,30 @@ int tree_flatten_device(DeviceContext &ctx, const Element *d_el, int64_t ne, con
     return FCG_NORMAL_END;
 }
 
+int tree_nodes_to_host(DeviceContext &ctx, Model &M, std::string &err) {
+    TF_CK(cudaSetDevice(ctx.device));
+    Bufs B;  // its stream
+    TF_CK(cudaStreamCreateWithFlags(&B.s, cudaStreamNonBlocking));
+    const DeviceNodes &d = *M.d_nodes;
+    const size_t nn = (size_t)M.n_nodes, np = (size_t)M.n_panels;
+    auto download = [&](auto &v, const auto *q, size_t n) -> cudaError_t {
+        v.resize(n);
+        return cudaMemcpyAsync(v.data(), q, n * sizeof(*q), cudaMemcpyDeviceToHost, B.s);
+    };
+    TF_CK(download(M.type, d.type, nn));
+    TF_CK(download(M.leaf_diel, d.leaf_diel, np));
+    TF_CK(download(M.left, d.left, nn));
+    TF_CK(download(M.right, d.right, nn));
+    TF_CK(download(M.leaf_first, d.leaf_first, nn));
+    TF_CK(download(M.leaf_count, d.leaf_count, nn));
+    TF_CK(download(M.vert, d.vert, 9 * nn));
+    TF_CK(download(M.cent, d.cent, 3 * nn));
+    TF_CK(download(M.norm, d.norm, 3 * nn));
+    TF_CK(download(M.area, d.area, nn));
+    TF_CK(download(M.maxside, d.maxside, nn));
+    TF_CK(cudaStreamSynchronize(B.s));
+    M.d_nodes.reset();
+    return FCG_NORMAL_END;
+}
+
 }  // namespace fcg

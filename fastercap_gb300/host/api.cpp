@@ -67,6 +67,15 @@ int model_build_device_links(DeviceContext *dev, const char *path, const fcg_bui
                              char *err, size_t err_len) {
     return build_on(dev, path, opt, true, nodes_too, out, err, err_len);
 }
+
+int model_nodes_to_host(DeviceContext *dev, fcg_model *m, std::string &err) {
+    try {
+        return m->m.d_nodes ? tree_nodes_to_host(*dev, m->m, err) : FCG_NORMAL_END;
+    } catch (std::bad_alloc &) {
+        err = "out of memory";
+        return FCG_OUT_OF_MEMORY;
+    }
+}
 }  // namespace fcg
 
 extern "C" int fcg_model_build_on(fcg_context *ctx, const char *path, const fcg_build_options *opt, fcg_model **out,

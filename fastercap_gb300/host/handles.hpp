@@ -18,6 +18,8 @@ namespace fcg {
 // memory (the model's arrays then point there); host/api.cpp
 int model_build_device_links(DeviceContext *dev, const char *path, const fcg_build_options *opt, bool nodes_too, fcg_model **out, char *err,
                              size_t err_len);
+// node arrays that such a model left in device memory go to its host vectors
+int model_nodes_to_host(DeviceContext *dev, fcg_model *m, std::string &err);
 }  // namespace fcg
 
 #endif

@@ -79,8 +79,8 @@ struct Model {
     // (BuildOptions::links_on_device); link_src is then empty
     std::shared_ptr<int32_t> d_link_src;
     // the node and leaf arrays in device memory when the build left them there
-    // (BuildOptions::nodes_on_device); the vectors of the same names, cond,
-    // maxside_idx and leaf_node are then empty
+    // (BuildOptions::nodes_on_device), until tree_nodes_to_host; the vectors of
+    // the same names are then empty, and cond, maxside_idx and leaf_node stay so
     std::unique_ptr<DeviceNodes> d_nodes;
     // leaves
     std::vector<int32_t> leaf_node;                // node of every leaf

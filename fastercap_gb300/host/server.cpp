@@ -93,7 +93,9 @@ static int count_conductors(const fcg_model_arrays &a) {
 }
 
 // build a file job's model on the server's GPU (mesh refinement and link
-// construction on the device), then wait until its footprint may be admitted
+// construction on the device), then wait until its footprint may be admitted.
+// A job that has to wait does so with its node arrays (102 bytes a node, which
+// no footprint counts) in host memory.
 static int build_file_job(fcg_server *s, Job *j) {
     double t0 = now_ms();
     char ebuf[512] = {0};
@@ -107,7 +109,14 @@ static int build_file_job(fcg_server *s, Job *j) {
     j->n_cond = count_conductors(j->a);
     j->footprint = fcg::problem_estimate_bytes(j->a, j->precision, j->n_cond, s->iterations_hint);
     std::unique_lock<std::mutex> lk(s->mu);
-    s->cv_admit.wait(lk, [&] { return j->cancel || s->solving == 0 || s->in_use + j->footprint <= s->budget; });
+    auto go = [&] { return j->cancel || s->solving == 0 || s->in_use + j->footprint <= s->budget; };
+    if (!go()) {
+        lk.unlock();
+        if ((r = fcg::model_nodes_to_host(s->ctx, j->model, j->error)) != FCG_NORMAL_END) return r;
+        fcg_model_arrays_get(j->model, &j->a);
+        lk.lock();
+        s->cv_admit.wait(lk, go);
+    }
     if (j->cancel) {
         j->footprint = 0;
         j->error = "job cancelled before its solve";
