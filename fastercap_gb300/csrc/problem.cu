@@ -688,16 +688,17 @@ __global__ void __launch_bounds__(256) k_fill_far(const int32_t *__restrict__ ro
     };
     const int r1 = row_split[blockIdx.x + 1];
     for (int row = row_split[blockIdx.x] + warp; row < r1; row += 8) {
-        const int s = (int)ptr[row], e = (int)ptr[row + 1];
-        for (int base = s; base < e; base += 32) {
-            const int l = base + lane;
+        // unsigned: the pass after the last of 2^31 - 1 links starts beyond them
+        const unsigned s = (unsigned)ptr[row], e = (unsigned)ptr[row + 1];
+        for (unsigned base = s; base < e; base += 32) {
+            const unsigned l = base + lane;
             const int band = l < e ? (int)(src[l] >> kBandShift) : 0;
             const int cls = band == 0 ? -1 : (band == 4 ? 0 : (band == 1 ? 2 : 1));
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 const unsigned m = __ballot_sync(0xffffffffu, cls == c);
                 if (!m) continue;
-                if (cls == c) qu[c][cnt[c] + __popc(m & ((1u << lane) - 1u))] = make_int2(l, row);
+                if (cls == c) qu[c][cnt[c] + __popc(m & ((1u << lane) - 1u))] = make_int2((int)l, row);
                 cnt[c] += __popc(m);
                 __syncwarp();
                 if (cnt[c] >= 32) {
@@ -1901,8 +1902,8 @@ __global__ void __launch_bounds__(256, K >= 16 ? 4 : (K >= 8 ? 6 : 7))
         int l = s + li;
         // the next row's link words (up to 1024 links) into L2
         auto prefetch_next = [&]() {
-            const int o = ns + 32 * lane;
-            if (o < ne) {
+            const unsigned o = (unsigned)ns + 32u * lane;  // may lie beyond 2^31 (and the row)
+            if (o < (unsigned)ne) {
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(coef + o));
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(src + o));
             }
