@@ -1913,14 +1913,14 @@ __global__ void __launch_bounds__(256, K >= 16 ? 4 : (K >= 8 ? 6 : 7))
                 // groups of four links are summed plainly, then added to the
                 // compensated sums; of a slot's last three, two are such a
                 // group and the third is its own update
-                for (; l + 7 * LPW < e; l += 8 * LPW) {
+                for (; (unsigned)l + 7u * LPW < (unsigned)e; l += 8 * LPW) {
                     float c[8];
                     float4 q[8];
                     load_links<8, LPL, LPW, true>(src, coef, Q4, l, e, ri, c, q);
                     link_add4(acc, c, q);
                     link_add4(acc, c + 4, q + 4);
                 }
-                for (; l + 3 * LPW < e; l += 4 * LPW) {
+                for (; (unsigned)l + 3u * LPW < (unsigned)e; l += 4 * LPW) {
                     float c[4];
                     float4 q[4];
                     load_links<4, LPL, LPW, true>(src, coef, Q4, l, e, ri, c, q);
@@ -1936,7 +1936,7 @@ __global__ void __launch_bounds__(256, K >= 16 ? 4 : (K >= 8 ? 6 : 7))
             } else {
                 // below 16 columns every link is an update of its own
                 if constexpr (K >= 8) {
-                    for (; l + 3 * LPW < e; l += 4 * LPW) {
+                    for (; (unsigned)l + 3u * LPW < (unsigned)e; l += 4 * LPW) {
                         float c[4];
                         float4 q[4];
                         load_links<4, LPL, LPW, true>(src, coef, Q4, l, e, ri, c, q);
