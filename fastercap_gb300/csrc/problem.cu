@@ -2472,13 +2472,11 @@ __global__ void k_reduce_seg(int nvec, int ks, int G, int nch, const double *__r
     if (lane == 0) out[sidx * ostride_s + j * ostride_j] = sum;
 }
 
-// one previous rotation applied to (t1, t2), every product rounded before
-// the sum (no contraction: the chain below forms rot_hi's two products apart)
+// a previous rotation's (t1, t2) -> (c t1 - s t2, c t2 + s t1): its first entry,
+// every product rounded before the sum (no contraction: the second entry is
+// the chain of step_end_warp, which forms the two products apart)
 __device__ __forceinline__ double rot_lo(double c, double s, double t1, double t2) {
     return __dsub_rn(__dmul_rn(c, t1), __dmul_rn(s, t2));
-}
-__device__ __forceinline__ double rot_hi(double c, double s, double t1, double t2) {
-    return __dadd_rn(__dmul_rn(c, t2), __dmul_rn(s, t1));
 }
 
 // out[r][j] = v[r][j] / hn[solve of (j, r)] for active solves, out = out_fixed
