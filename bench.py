@@ -70,9 +70,9 @@ MULTI = {
 # dram__bytes_write.sum) from one ncu capture of the same kernel and
 # workload, with the summary that records the capture
 LINK_TRAFFIC = {
-    "sphere_327680": (534.116864e6 + 4.707072e6, "profiles/sphere_327680_kernels_full.md"),  # k_spmv32<1, 16>
-    "crossing8x8_slab": (677.425664e6 + 7.629056e6, "profiles/crossing8x8_slab_spmv32_multi.md"),  # k_spmv32_multi<16>
-    "serving_request0": (282.506752e6 + 16.958976e6, "profiles/serving_request0_kernels.md"),  # k_spmv32_multi<24>
+    "sphere_327680": (538.474752e6 + 4.422656e6, "profiles/sphere_327680_kernels_full.md"),  # k_spmv32<1, 8>
+    "crossing8x8_slab": (698.999040e6 + 29.188352e6, "profiles/crossing8x8_slab_spmv32_multi.md"),  # k_spmv32_multi<16>
+    "serving_request0": (278.722816e6 + 39.810304e6, "profiles/serving_request0_kernels.md"),  # k_spmv32_multi<24>
 }
 
 
@@ -565,11 +565,11 @@ def serving_roofline(ctx, path):
             "achieved": ach, "peak": peak, "unit": "GB/s", "frac": (ach / peak) if ach else None, "peak_source": peak_kind,
             "traffic": LINK_TRAFFIC["serving_request0"][0], "traffic_source": LINK_TRAFFIC["serving_request0"][1],
             "launches": int(st["link_launches"]), "bytes_per_launch": b, "avg_launch_ms": ms,
-            "gather_path": "bound by the L1 gather path, not HBM: L1 LSU wavefronts 63.5 pct of peak, issue 60 pct, "
-                           "DRAM 12 pct (ncu, " + LINK_TRAFFIC["serving_request0"][1] + ")",
-            "krylov": "k_dots and k_update (about 27 pct of the request's device time) run FP32-pair arithmetic "
+            "gather_path": "bound by the L1 gather path, not HBM: L1 LSU wavefronts 70 pct of peak, issue 56 pct, "
+                           "DRAM 15 pct (ncu, " + LINK_TRAFFIC["serving_request0"][1] + ")",
+            "krylov": "k_dots and k_update (about 29 pct of the request's device time) run FP32-pair arithmetic "
                       "on a basis stored as FP32 pairs and are bound by HBM: at Arnoldi step 40 they move 1.20 and "
-                      "1.22 GB in 210 and 204 us, 0.84 and 0.89 of the measured copy bandwidth (ncu, "
+                      "1.22 GB in 202 and 195 us, 0.87 and 0.92 of the measured copy bandwidth (ncu, "
                       + LINK_TRAFFIC["serving_request0"][1] + ")"}
 
 
