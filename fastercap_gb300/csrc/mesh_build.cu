@@ -188,8 +188,9 @@ __device__ __forceinline__ void emit_splits(LevelHead *head, int64_t ne, int f, 
 // together (one round: at once, the queue would only add a round). Levels of
 // 42 / 120 million pairs in all 2720 / 6335 -> 2063 / 4575 us with the 16-byte
 // loads of PairElement (without the queue 2420 / 5880, the queue alone 2435 /
-// 5320); a small level 11.7 -> 7.7. What is left is latency at 24 warps an SM:
-// 20 (no spills) 2277 / 5265, 32 2111 / 4504. Four pairs a lane with one claim
+// 5320); a small level 11.7 -> 7.7. What is left is the FP64 pipe (areas and
+// sides; 55 % active in the longest level) and latency at 24 warps an SM: 20 (no
+// spills) 2277 / 5265, 32 2111 / 4504. Four pairs a lane with one claim
 // (218 -> 300 us a level of 4M pairs) and one claim a CTA (2842 / 7243) were
 // slower. A small level is bound by its launches: three kernels a level and a
 // wait for the host every few levels, instead of nine and one each: a 528-panel
